@@ -858,6 +858,12 @@ __device__ __forceinline__ void stage_segments(const FusedArgs& A, WarpStage<R>&
   }
 }
 
+}  // namespace bbhx
+
+#include "direct_panel.cuh"
+
+namespace bbhx {
+
 // One WARP item = (data tile of FD_TILE bins, binary).  Items are enumerated tile-major and
 // claimed in increasing order (claim_item), so the warps in flight work on the same data tile
 // for different binaries and share it through L2.
@@ -876,12 +882,12 @@ __device__ __forceinline__ void stage_segments(const FusedArgs& A, WarpStage<R>&
 // uniform (A.grid), with its state in RS.
 template <bool MIXED, typename R, bool GH = false, bool REC = false>
 __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, WarpStage<R>& S,
-                                           RecStage* RS, int lane) {
+                                           RecStage* RS, PanelStage* PS, int lane) {
   const long long BML = A.qstride;
   const int L = A.L;
   bool uni = false;
   double gk0 = 0.0, gdf = 0.0;
-  if (REC && A.grid != nullptr) {
+  if (!MIXED && A.grid != nullptr) {
     const unsigned ok = A.grid->ok & 7u;
     if (ok) {
       uni = true;
@@ -902,6 +908,26 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
         P[0] = 0.0; P[1] = 0.0; P[2] = 0.0;
       }
       return;
+    }
+    if constexpr (!MIXED && !GH) {
+      if (uni) {
+        const int kk = (lane < A.M) ? A.segtab[q * A.M + lane].x : 0;
+        double dr = 0.0, di = 0.0, hh = 0.0;
+        panel_item(A, S, *PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, gk0, gdf, dr, di, hh);
+        for (int o = 16; o > 0; o >>= 1) {
+          dr += __shfl_xor_sync(0xffffffffu, dr, o);
+          di += __shfl_xor_sync(0xffffffffu, di, o);
+          hh += __shfl_xor_sync(0xffffffffu, hh, o);
+        }
+        if (lane == 0) {
+          double* P = A.partials + 3 * q;
+          P[0] = dr;
+          P[1] = di;
+          P[2] = hh;
+        }
+        __syncwarp();
+        return;
+      }
     }
     // ---- stage this tile's segments for every mode
     if (REC && lane < FD_MAXM) RS->next_chunk[lane] = -1;
@@ -1242,26 +1268,27 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
 
 // Shared memory of the fused kernels: FD_WARPS WarpStage slices, then (FP64 form, phase
 // recurrence) FD_WARPS RecStage slices.
-template <bool MIXED>
+template <bool MIXED, bool GH = false>
 constexpr size_t fused_smem_bytes() {
   using R = typename std::conditional<MIXED, float, double>::type;
-  return FD_WARPS * (sizeof(WarpStage<R>) + (MIXED ? 0 : sizeof(RecStage)));
+  return FD_WARPS * (sizeof(WarpStage<R>) +
+                     (MIXED ? 0 : GH ? sizeof(RecStage) : sizeof(PanelStage)));
 }
 
 template <bool MIXED, bool GH = false>
 __global__ void __launch_bounds__(FD_WARPS * 32, MIXED ? 4 : 3) k_direct_fused(FusedArgs A) {
   static_assert(!(MIXED && GH), "d lnL / d h is written by the FP64 form only");
   using R = typename std::conditional<MIXED, float, double>::type;
-  constexpr bool REC = !MIXED;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   WarpStage<R>& S = reinterpret_cast<WarpStage<R>*>(smem_raw)[warp];
-  RecStage* RS = REC ? reinterpret_cast<RecStage*>(smem_raw + FD_WARPS * sizeof(WarpStage<R>)) + warp
-                     : nullptr;
+  unsigned char* extra = smem_raw + FD_WARPS * sizeof(WarpStage<R>);
+  RecStage* RS = reinterpret_cast<RecStage*>(extra) + warp;
+  PanelStage* PS = reinterpret_cast<PanelStage*>(extra) + warp;
   const long long nitems = (long long)A.ntiles * A.B;
   for (long long q = claim_item(A.next, lane); q < nitems; q = claim_item(A.next, lane))
-    fused_item<MIXED, R, GH, REC>(A, q, S, RS, lane);
+    fused_item<MIXED, R, GH, GH>(A, q, S, RS, PS, lane);
 }
 
 // Several independent problems (groups: own data stream, grid length L, mode count M,
@@ -1335,7 +1362,6 @@ __global__ void __launch_bounds__(FD_WARPS * 32, (MIXED && !HET) ? 4 : 3)
     k_uneven(const MultiArgs* __restrict__ MA, const HetMulti* __restrict__ HM, int slot,
              unsigned long long* next) {
   using R = typename std::conditional<MIXED, float, double>::type;
-  constexpr bool REC = !MIXED;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ FusedArgs gcur[FD_WARPS];
   __shared__ HetArgs hcur[FD_WARPS];
@@ -1343,7 +1369,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32, (MIXED && !HET) ? 4 : 3)
   const int warp = threadIdx.x >> 5;
   unsigned char* mine = smem_raw + (size_t)warp * slot;
   WarpStage<R>& S = *reinterpret_cast<WarpStage<R>*>(mine);
-  RecStage* RS = REC ? reinterpret_cast<RecStage*>(mine + sizeof(WarpStage<R>)) : nullptr;
+  PanelStage* PS = reinterpret_cast<PanelStage*>(mine + sizeof(WarpStage<R>));
   const long long nh = HM->woff[HM->ngroups];
   const long long total = nh + MA->off[MA->ngroups];
   int g = -1, hg = -1;
@@ -1373,7 +1399,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32, (MIXED && !HET) ? 4 : 3)
         for (int i = lane; i < n8; i += 32) dst[i] = src[i];
         __syncwarp();
       }
-      fused_item<MIXED, R, false, REC>(gcur[warp], qd - MA->off[g], S, RS, lane);
+      fused_item<MIXED, R>(gcur[warp], qd - MA->off[g], S, nullptr, PS, lane);
     }
   }
 }
@@ -1422,14 +1448,14 @@ __global__ void k_fused_reduce_multi(const MultiArgs* __restrict__ MA) {
 // out: d_h[b], h_h[b] complex (device).  One warp per binary: lane l sums tiles l, l+32, ...
 // of the binary's support, then a fixed shuffle tree; the order is the same on every run.
 __global__ void k_fused_reduce(const double* partials, const int* sup_start, const int* sup_len,
-                               int B, double* d_h, double* h_h) {
+                               int B, int tile, double* d_h, double* h_h) {
   const int lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
   for (int b = blockIdx.x * wpb + (threadIdx.x >> 5); b < B; b += gridDim.x * wpb) {
     double a = 0, c = 0, h = 0;
     int s0 = sup_start[b], n = sup_len[b];
     if (n > 0) {
-      int tlo = s0 / FD_TILE, thi = (s0 + n - 1) / FD_TILE;
+      int tlo = s0 / tile, thi = (s0 + n - 1) / tile;
       for (int t = tlo + lane; t <= thi; t += 32) {
         const double* P = partials + 3 * ((long long)t * B + b);
         a += P[0];
@@ -1474,6 +1500,16 @@ unsigned resident_grid(K kernel, size_t smem, long long nitems) {
   }
   const long long want = (nitems + FD_WARPS - 1) / FD_WARPS;
   return (unsigned)std::max<long long>(1, std::min<long long>(want, (long long)per_sm * sm_count()));
+}
+
+// Data bins per work item of a single-problem launch: the largest tile that still gives every
+// resident warp several items, since an item of a low-frequency tile takes many times the
+// average (few binaries: the call ends when its slowest item does).
+inline int fused_tile(int N, int B) {
+  const long long warps = (long long)sm_count() * 3 * FD_WARPS;
+  int tile = FD_TILE;
+  while (tile > 256 && ((long long)N + tile - 1) / tile * B < 8 * warps) tile >>= 1;
+  return tile;
 }
 
 int direct_fused_gh(cplx* gh, const long long* gh_off, double* d_h, double* h_h,
@@ -1529,7 +1565,7 @@ int direct_fused_gh(cplx* gh, const long long* gh_off, double* d_h, double* h_h,
     A.gh_off = gh_off;
     A.grid = grid;
     A.next = next;
-    const size_t sm = fused_smem_bytes<false>();
+    const size_t sm = fused_smem_bytes<false, true>();
     st = cuda_status(cudaFuncSetAttribute(k_direct_fused<false, true>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
                      "cudaFuncSetAttribute(k_direct_fused)");
@@ -1542,7 +1578,7 @@ int direct_fused_gh(cplx* gh, const long long* gh_off, double* d_h, double* h_h,
     }
   }
   if (!st && d_h != nullptr && h_h != nullptr) {
-    k_fused_reduce<<<grid_for(32LL * nb, 128), 128, 0, s>>>(part, start + b0, len + b0, nb,
+    k_fused_reduce<<<grid_for(32LL * nb, 128), 128, 0, s>>>(part, start + b0, len + b0, nb, FD_TILE,
                                                             d_h + 2LL * b0, h_h + 2LL * b0);
     st = launch_status("k_fused_reduce");
   }
@@ -1944,8 +1980,9 @@ int bbhx_direct_like_fused(double* d_h, double* h_h, const double* data_freqs, c
   BBHX_REQUIRE(num_modes <= FD_MAXM, "num_modes must be <= 6");
   if (num_bin_all == 0) return OK;
   cudaStream_t s = (cudaStream_t)stream;
-  int ntiles = (data_length + FD_TILE - 1) / FD_TILE;
-  long long nitems = (long long)ntiles * num_bin_all;
+  const int tile = fused_tile(data_length, num_bin_all);
+  const int ntiles = (data_length + tile - 1) / tile;
+  const long long nitems = (long long)ntiles * num_bin_all;
   int* sup = nullptr;
   double* part = nullptr;
   int2* segtab = nullptr;
@@ -1963,7 +2000,7 @@ int bbhx_direct_like_fused(double* d_h, double* h_h, const double* data_freqs, c
   if (!st) {
     k_tile_segments<<<grid_for(nitems * num_modes, 256, sm_count() * 64), 256, 0, s>>>(
         segtab, x, data_freqs, sup, sup + num_bin_all, num_bin_all, num_modes, length, ntiles,
-        FD_TILE);
+        tile);
     st = launch_status("k_tile_segments");
   }
   if (!st) {
@@ -1985,7 +2022,7 @@ int bbhx_direct_like_fused(double* d_h, double* h_h, const double* data_freqs, c
     A.M = num_modes;
     A.L = length;
     A.ntiles = ntiles;
-    A.tile = FD_TILE;
+    A.tile = tile;
     A.partials = part;
     A.segtab = segtab;
     A.d_h = d_h;
@@ -2015,7 +2052,7 @@ int bbhx_direct_like_fused(double* d_h, double* h_h, const double* data_freqs, c
   }
   if (!st) {
     k_fused_reduce<<<grid_for(32LL * num_bin_all, 128), 128, 0, s>>>(part, sup, sup + num_bin_all,
-                                                              num_bin_all, d_h, h_h);
+                                                                     num_bin_all, tile, d_h, h_h);
     st = launch_status("k_fused_reduce");
   }
   pool_free(sup, s);
