@@ -8,9 +8,17 @@
 // observation of months, so the residual phases stay below kPanelDelta over hundreds of bins
 // and Q_c is a polynomial of degree 7 to ~5e-14: it is built from the modes' exact values at
 // eight nodes (lanes = node x mode), and a bin then costs three polynomials and one carrier
-// product for all modes together instead of seven cubics and three rotations per mode (75 FP64
-// instructions per bin for six modes, against 306).  Where the modes do not stay together (a
-// few 1e-3 of the band) the bins are evaluated one by one.
+// product for all modes together instead of seven cubics and three rotations per mode: 101 FP64
+// instructions per bin for six modes with everything included, against 306.  Where the modes do
+// not stay together (1-4 % of the band of a 1-yr stream) the bins are evaluated one by one.
+//
+// What bounds it (B = 1024, 1 yr, six modes, L = 1024; 86.4 ms before the panels, 26 ms now): the
+// FP64 pipe is 50 % busy counted at 2 cycles an instruction, but a DFMA that reads three
+// registers anew takes 3 (40.7 of 64 lanes per clock measured, 53 in the order of panel_bins), so
+// the pipe is two thirds busy, the shared-memory and load path 60 %, issue 50 %.  Data in L1
+// instead of L2: no change.  A second resident CTA's worth of warps (16 per SM at 128 registers)
+// gains 3 % on large batches and loses 5 % on small ones; dropping negligible powers at run time,
+// unrolled per degree or in a short loop over channels: 3-5 % slower.
 #pragma once
 
 namespace bbhx {
@@ -18,19 +26,20 @@ namespace bbhx {
 constexpr int kPanelNodes = 8;
 // Residual phase over a panel, linear and quadratic part (rad): the degree-7 interpolation error
 // of e^{i (delta s + q s^2)} is ~2e-13 at both limits.  Amplitude and transfer functions add to
-// it; panel_smooth checks the coefficients themselves.
-constexpr double kPanelDelta = 0.15;
-constexpr double kPanelQuad = 1.5e-3;
+// it; panel_degree checks the coefficients themselves.
+constexpr float kPanelDelta = 0.15f;
+constexpr float kPanelQuad = 1.5e-3f;
 constexpr float kPanelTail = 1.6e-8f;  // largest |c_6|, |c_7| against the largest coefficient
 constexpr int kPanelBins = 1024;       // longest panel
 constexpr int kPanelMinBins = 24;      // below this the nodes cost more than the bins
 constexpr int kPanelDirect = 128;      // bins evaluated one by one at a time
+constexpr int kPanelRing = 4;          // segments of a mode in shared memory (power of two)
 
 // Nodes +-t_q on [-1, 1]: Chebyshev points rounded to multiples of 1/128, so that a node's bin
 // position is exact.  Row p of kPanelCoef: coefficient of s^p = sum_q row[q] (F(t_q) + F(-t_q))
 // for even p, (F(t_q) - F(-t_q)) for odd p.
 __device__ const double kPanelTau[4] = {0.984375, 0.828125, 0.5625, 0.1953125};
-__device__ const double kPanelCoef[kPanelNodes][4] = {
+__device__ const __align__(16) double kPanelCoef[kPanelNodes][4] = {
     {-0.024057555333062423, 0.0863143273345492, -0.188962393279747, 0.6267056212782602},
     {-0.02443942129073008, 0.10422862168700281, -0.3359331436084391, 3.2087327809446924},
     {0.741768143135053, -2.624550413047438, 5.4240838960065085, -3.5413016260941235},
@@ -40,20 +49,55 @@ __device__ const double kPanelCoef[kPanelNodes][4] = {
     {2.906394550207518, -7.380004179614286, 7.454222650728741, -2.980613021321973},
     {2.9525277970362085, -8.91170316028895, 13.251951379073317, -15.260738669168502}};
 
-// Per-warp shared memory of the panel path beside the staged segments.
+// Per-warp shared memory of the panel path.  Segment k of mode m (9 quantities x (y, c1, c2, c3))
+// sits in ring slot k mod 4, knot j in slot j mod 8.
 struct alignas(16) PanelStage {
+  double co[FD_MAXM][kPanelRing][FD_NC];
+  double x[FD_MAXM][8];
   double2 C[3][kPanelNodes];   // polynomial coefficients of Q_c in s
   double F[kPanelNodes][6];    // Q_c at the nodes (0..3: +t_q, 4..7: -t_q)
+  double2 E[32];               // e^{i b lane}
+  double xk[FD_MAXM];          // knot of each mode's segment in this panel
+  double kb[FD_MAXM];          // its position in bins
+  float4 sl[FD_MAXM];          // phase slope in rad per bin, x + y t + z t^2 at t bins after it
   double lo[FD_MAXM], hi[FD_MAXM];  // first and last knot of each mode
   float per[FD_MAXM];          // (L - 1) / log(hi / lo)
-  int kl[FD_MAXM];             // staged segment of each mode in this panel, -1: contributes nothing
+  int slot[FD_MAXM];           // ring slot of each mode's segment, -1: contributes nothing
 };
 
-// First bin i in [0, N] with fl((k0 + i) df) >= x (the grid frequency, see GridInfo).
-__device__ __forceinline__ int first_bin_at(double x, double k0, double df, int N) {
-  int i = (int)fmin(fmax(ceil(x / df) - k0, 0.0), (double)N);
-  while (i > 0 && __dmul_rn(k0 + (double)(i - 1), df) >= x) --i;
-  while (i < N && __dmul_rn(k0 + (double)i, df) < x) ++i;
+// Quantity p (0 amplitude, 1 phase, 2 t(f), 3..8 transfer) of a staged segment.
+struct PanelCoef {
+  const double* seg;
+  double x;
+  __device__ __forceinline__ double xk() const { return x; }
+  __device__ __forceinline__ void get(int p, double* c) const {
+    const double2 lo = *reinterpret_cast<const double2*>(seg + 4 * p);
+    const double2 hi = *reinterpret_cast<const double2*>(seg + 4 * p + 2);
+    c[0] = lo.x; c[1] = lo.y; c[2] = hi.x; c[3] = hi.y;
+  }
+};
+
+// 8 bytes from global to shared memory without a register in between.
+__device__ __forceinline__ void copy8_async(double* dst, const double* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// First bin i in [0, N] with fl((k0 + i) df) >= x (the grid frequency, see GridInfo), from the
+// knot's position xb = x / df - k0 in bins (good to ~1e-9: only near an integer the frequencies
+// themselves are compared).
+__device__ __forceinline__ int first_bin_at(double x, double xb, double k0, double df, int N) {
+  const double c = ceil(xb);
+  int i = (int)fmin(fmax(c, 0.0), (double)N);
+  if (!(fabs(xb - rint(xb)) > 1e-6)) {
+    while (i > 0 && __dmul_rn(k0 + (double)(i - 1), df) >= x) --i;
+    while (i < N && __dmul_rn(k0 + (double)i, df) < x) ++i;
+  }
   return i;
 }
 
@@ -78,26 +122,50 @@ __device__ __forceinline__ int segment_guess(const double* __restrict__ xr, int 
   return a - 1;
 }
 
+// t(f) gate over a whole segment from the control points of its cubic (their hull holds it): 1 all
+// inside the observation window, 2 all outside, 0 undecided (per-bin gate).
+__device__ __forceinline__ int hull_gate(const double* c, double h, double ts, double te) {
+  const double a = c[1] * h, q = c[2] * h * h;
+  const double p1 = c[0] + a * (1.0 / 3.0);
+  const double p2 = c[0] + (2.0 * a + q) * (1.0 / 3.0);
+  const double p3 = c[0] + a + q + c[3] * h * h * h;
+  const double lo = fmin(fmin(c[0], p1), fmin(p2, p3));
+  const double hi = fmax(fmax(c[0], p1), fmax(p2, p3));
+  const double eps = 1e-6;  // s: far above the rounding of t(f), as in segment_gate
+  if (!(lo == lo) || !(hi == hi)) return 0;
+  if (lo >= ts + eps && (te <= 0.0 || hi <= te - eps)) return 1;
+  if (hi < ts - eps || (te > 0.0 && lo > te + eps)) return 2;
+  return 0;
+}
+
+// Order-preserving integer of a float and back (warp max / min by integer reductions).
+__device__ __forceinline__ int order_key(float v) {
+  const int b = __float_as_int(v);
+  return b ^ ((b >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float order_value(int k) {
+  return __int_as_float(k ^ ((k >> 31) & 0x7fffffff));
+}
+
 // Whether the panel's polynomials have converged: the two highest coefficients of every channel
 // lie below kPanelTail of its largest one (lanes = channel x power).
 __device__ __forceinline__ bool panel_smooth(const PanelStage& PS, int lane) {
-  const int ch = min(lane >> 3, 2), p = lane & 7;
-  const double2 c = PS.C[ch][p];
-  const double v = fabs(c.x) + fabs(c.y);
-  double top = v;
+  const double2 c = PS.C[min(lane >> 3, 2)][lane & 7];
+  const float v = (float)(fabs(c.x) + fabs(c.y));
+  float top = v;
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
-  return !__any_sync(0xffffffffu, p >= 6 && v > kPanelTail * top);
+  for (int o = 4; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+  return !__any_sync(0xffffffffu, (lane & 7) >= 6 && v > kPanelTail * top);
 }
 
 // Q_c at the panel's nodes, then its polynomial coefficients into PS.C.  Lane = (node, mode
 // group): lanes 8 g .. 8 g + 7 take the nodes of modes g and g + 4.  kc = k0 + ia; the node
 // sits `off` bins after ia (exact), its phase is evaluated at k df with the error-free product
 // and compensated sums of rot_anchor, and the carrier b * off is taken off before the reduction.
-__device__ __forceinline__ void panel_nodes(const WarpStage<double>& S, PanelStage& PS, int M,
-                                            int lane, double kc, double center, double half,
-                                            double df, double b, double tau, const double* row) {
+__device__ __forceinline__ void panel_nodes(PanelStage& PS, int M, int lane, double kc,
+                                            double center, double half, double df, double b) {
   const int node = lane & 7, grp = lane >> 3;
+  const double tau = (lane & 4) ? -kPanelTau[lane & 3] : kPanelTau[lane & 3];
   const double off = fma(half, tau, center);
   const double kd = kc + off;
   const double p = __dmul_rn(kd, df);
@@ -106,11 +174,11 @@ __device__ __forceinline__ void panel_nodes(const WarpStage<double>& S, PanelSta
   const double lo = fma(b, off, -hi);
   double F[6] = {0, 0, 0, 0, 0, 0};
   for (int m = grp; m < M; m += 4) {
-    const int k = PS.kl[m];
-    if (k < 0) continue;
-    const double u = __dsub_rn(p, S.x[m][k]);
+    const int sl = PS.slot[m];
+    if (sl < 0) continue;
+    const PanelCoef src{PS.co[m][sl], PS.xk[m]};
+    const double u = __dsub_rn(p, src.x);
     double c[4];
-    const SmemCoef src{S, m, k};
     src.get(1, c);
     double t = u * fma(fma(c[3], u, c[2]), u, c[1]);
     t = fma(fma(fma(3.0 * c[3], u, 2.0 * c[2]), u, c[1]), pe, t);
@@ -157,6 +225,9 @@ __device__ __forceinline__ void panel_nodes(const WarpStage<double>& S, PanelSta
   __syncwarp();
   // coefficient of s^node for components grp and grp + 4
   const double sg = (node & 1) ? -1.0 : 1.0;
+  const double2 r01 = __ldg(reinterpret_cast<const double2*>(kPanelCoef[node]));
+  const double2 r23 = __ldg(reinterpret_cast<const double2*>(kPanelCoef[node]) + 1);
+  const double row[4] = {r01.x, r01.y, r23.x, r23.y};
   double* C = reinterpret_cast<double*>(PS.C);
 #pragma unroll
   for (int r = 0; r < 2; ++r) {
@@ -171,8 +242,8 @@ __device__ __forceinline__ void panel_nodes(const WarpStage<double>& S, PanelSta
   __syncwarp();
 }
 
-// Sums over the panel's n bins from ia: hh += |w Q|^2, (zr, zi) = sum_i z_i R^(j) of the lane's
-// bins i = ia + lane + 32 j, with z = sum_c d~_c w Q_c, taken from the last bin down (Horner in
+// Sums over the panel's n bins from ia: hh += |w Q|^2, (zr, zi) = sum_j a_j R^j over the lane's
+// bins i = ia + lane + 32 j, a = sum_c d~_c w Q_c, taken from the last bin down (Horner in
 // R = e^{i 32 b}), so the carrier costs one complex product per bin.
 __device__ __forceinline__ void panel_bins(const FusedArgs& A, const PanelStage& PS, int ia, int n,
                                            double center, double inv_half, int lane, double Rr,
@@ -180,14 +251,13 @@ __device__ __forceinline__ void panel_bins(const FusedArgs& A, const PanelStage&
   zr = zi = 0.0;
   const double* wp = A.noise + ia + lane;
   const double2* dp = reinterpret_cast<const double2*>(A.data) + ia + lane;
+  const double s0 = ((double)lane - center) * inv_half, ds = 32.0 * inv_half;
   for (int j0 = ((n - 1) >> 7) << 2; j0 >= 0; j0 -= FD_K) {
+    const bool full = n - 32 * j0 >= 32 * FD_K;  // every lane has all its bins
     double s[FD_K], ar[FD_K], ai[FD_K];
-    bool ok[FD_K];
 #pragma unroll
     for (int j = 0; j < FD_K; ++j) {
-      const int i = lane + 32 * (j0 + j);
-      ok[j] = i < n;
-      s[j] = ok[j] ? ((double)i - center) * inv_half : 0.0;
+      s[j] = fma((double)(j0 + j), ds, s0);
       ar[j] = 0.0;
       ai[j] = 0.0;
     }
@@ -195,11 +265,21 @@ __device__ __forceinline__ void panel_bins(const FusedArgs& A, const PanelStage&
     for (int ch = 0; ch < 3; ++ch) {
       double w[FD_K], qr[FD_K], qi[FD_K];
       double2 d[FD_K];
+      const double* wc = wp + (long long)ch * A.N + 32 * j0;
+      const double2* dc = dp + (long long)ch * A.N + 32 * j0;
+      if (full) {
 #pragma unroll
-      for (int j = 0; j < FD_K; ++j) {
-        const long long o = (long long)ch * A.N + 32 * (j0 + j);
-        w[j] = ok[j] ? __ldg(wp + o) : 0.0;
-        d[j] = ok[j] ? __ldg(dp + o) : make_double2(0.0, 0.0);
+        for (int j = 0; j < FD_K; ++j) {
+          w[j] = __ldg(wc + 32 * j);
+          d[j] = __ldg(dc + 32 * j);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < FD_K; ++j) {
+          const bool ok = lane + 32 * (j0 + j) < n;
+          w[j] = ok ? __ldg(wc + 32 * j) : 0.0;
+          d[j] = ok ? __ldg(dc + 32 * j) : make_double2(0.0, 0.0);
+        }
       }
       const double2 top = PS.C[ch][kPanelNodes - 1];
 #pragma unroll
@@ -211,10 +291,9 @@ __device__ __forceinline__ void panel_bins(const FusedArgs& A, const PanelStage&
       for (int p = kPanelNodes - 2; p >= 0; --p) {
         const double2 c = PS.C[ch][p];
 #pragma unroll
-        for (int j = 0; j < FD_K; ++j) {
-          qr[j] = fma(qr[j], s[j], c.x);
-          qi[j] = fma(qi[j], s[j], c.y);
-        }
+        for (int j = 0; j < FD_K; ++j) qr[j] = fma(qr[j], s[j], c.x);
+#pragma unroll
+        for (int j = 0; j < FD_K; ++j) qi[j] = fma(qi[j], s[j], c.y);
       }
 #pragma unroll
       for (int j = 0; j < FD_K; ++j) {
@@ -267,190 +346,266 @@ __device__ __forceinline__ void panel_scatter(const FusedArgs& A, const PanelSta
   }
 }
 
-// The n bins from ia one by one (lanes over bins), every mode behind its per-bin t(f) gate: runs
-// where a mode crosses the observation window or the modes' phases do not stay together.
-__device__ __forceinline__ void panel_direct(const FusedArgs& A, const WarpStage<double>& S,
-                                             const PanelStage& PS, int ia, int n, int lane,
-                                             double k0, double df, double ts, double te,
+// The n bins from ia one by one, G bins per lane at a time: runs where a mode crosses the
+// observation window (GATE: its t(f) decides bin by bin) or the modes' phases do not stay
+// together.
+template <int G, bool GATE>
+__device__ __forceinline__ void panel_direct(const FusedArgs& A, const PanelStage& PS, int b,
+                                             int ia, int n, int lane, double k0, double df,
                                              double& dr, double& di, double& hh) {
-  for (int i = ia + lane; i < ia + n; i += 32) {
-    const double f = __dmul_rn(k0 + (double)i, df);
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (int m = 0; m < A.M; ++m) {
-      const int k = PS.kl[m];
-      if (k >= 0) accumulate_bin_src(SmemCoef{S, m, k}, f, ts, te, acc);
-    }
-    bin_products(A, i, acc, dr, di, hh);
+  double ts = 0.0, te = 0.0;
+  if (GATE) {
+    ts = __ldg(A.t_start + b);
+    te = __ldg(A.t_end + b);
   }
-}
-
-// Bins [i0, i1) of binary b (inside its support) by one warp; kk = the segments of bin i0 in
-// lanes 0 .. M-1 (-1 before a mode's first knot, L-1 past its last).  Lane m walks mode m: its
-// segment, the first bin of the next one, its staged window of segments.  Per-lane partial sums
-// into dr, di, hh.
-__device__ __forceinline__ void panel_item(const FusedArgs& A, WarpStage<double>& S,
-                                           PanelStage& PS, int b, int i0, int i1, int kk,
-                                           int lane, double k0, double df, double& dr, double& di,
-                                           double& hh) {
-  constexpr int NSEG = WarpStage<double>::NSEG;
-  const int M = A.M, L = A.L;
-  const bool mine = lane < M;
-  const double ts = __ldg(A.t_start + b), te = __ldg(A.t_end + b);
-  const double tau = (lane & 4) ? -kPanelTau[lane & 3] : kPanelTau[lane & 3];
-  double row[4];
+#pragma unroll 1
+  for (int i = lane; i < n; i += 32 * G) {
+    double f[G], acc[G][6];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) row[q] = __ldg(&kPanelCoef[lane & 7][q]);
-  int k = kk, klo = 0, nst = 0, next = 0;
-  int i = i0;
-  // runs where the knots of all modes lie closer than kPanelMinBins bins on average
-  const double* xr = A.x + ((long long)b * M + (mine ? lane : 0)) * L;
-  double lo = 0.0, hi = 0.0;
-  float per = 0.0f;
-  if (mine) {
-    lo = __ldg(xr);
-    hi = __ldg(xr + L - 1);
-    per = (float)(L - 1) / logf((float)(hi / lo));
-    PS.lo[lane] = lo;
-    PS.hi[lane] = hi;
-    PS.per[lane] = per;
+    for (int j = 0; j < G; ++j) {
+      f[j] = __dmul_rn(k0 + (double)(ia + min(i + 32 * j, n - 1)), df);
+#pragma unroll
+      for (int c = 0; c < 6; ++c) acc[j][c] = 0.0;
+    }
+#pragma unroll 1
+    for (int m = 0; m < A.M; ++m) {
+      const int sl = PS.slot[m];
+      if (sl < 0) continue;
+      const PanelCoef src{PS.co[m][sl], PS.xk[m]};
+      double c[4], u[G], apr[G], api[G];
+      bool in[G];
+#pragma unroll
+      for (int j = 0; j < G; ++j) {
+        u[j] = f[j] - src.x;
+        in[j] = true;
+      }
+      if (GATE) {
+        src.get(2, c);
+#pragma unroll
+        for (int j = 0; j < G; ++j)
+          in[j] = tf_gate(fma(fma(fma(c[3], u[j], c[2]), u[j], c[1]), u[j], c[0]), ts, te);
+      }
+      src.get(1, c);
+#pragma unroll
+      for (int j = 0; j < G; ++j)
+        sincos_cw(fma(fma(fma(c[3], u[j], c[2]), u[j], c[1]), u[j], c[0]), &api[j], &apr[j]);
+      src.get(0, c);
+#pragma unroll
+      for (int j = 0; j < G; ++j) {
+        const double a = in[j] ? fma(fma(fma(c[3], u[j], c[2]), u[j], c[1]), u[j], c[0]) : 0.0;
+        apr[j] *= a;
+        api[j] *= a;
+      }
+#pragma unroll
+      for (int ch = 0; ch < 3; ++ch) {
+        src.get(3 + 2 * ch, c);
+        double e[4];
+        src.get(4 + 2 * ch, e);
+#pragma unroll
+        for (int j = 0; j < G; ++j) {
+          const double tr = fma(fma(fma(c[3], u[j], c[2]), u[j], c[1]), u[j], c[0]);
+          const double ti = fma(fma(fma(e[3], u[j], e[2]), u[j], e[1]), u[j], e[0]);
+          acc[j][2 * ch] += tr * apr[j] - ti * api[j];
+          acc[j][2 * ch + 1] -= tr * api[j] + ti * apr[j];
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < G; ++j)
+      if (i + 32 * j < n) bin_products(A, ia + i + 32 * j, acc[j], dr, di, hh);
   }
   __syncwarp();
-  for (;;) {
-    float dens = 0.0f;
-    if (mine && k >= 0 && k < L - 1) dens = (float)(df / (__ldg(xr + k + 1) - __ldg(xr + k)));
+}
+
+// Bins [i0, i1) of binary b (inside its support) by one warp; kk = the segments of bins i0 and
+// i1 - 1 in lanes 0 .. M-1 (-1 before a mode's first knot, L-1 past its last).  Lane m walks mode
+// m.  When a mode enters segment k its freed ring slot is refilled with segment k + 3 by
+// asynchronous copies, three entries ahead of their use.  Per-lane partial sums into dr, di, hh.
+__device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, int b, int i0,
+                                           int i1, int2 kk, int lane, double k0, double df,
+                                           double& dr, double& di, double& hh) {
+  const int M = A.M, L = A.L;
+  const bool mine = lane < M;
+  int k = mine ? kk.x : L - 1;
+  const int klast = mine ? min(kk.y, L - 2) : -1;  // last segment of the item
+  int i = i0;
+  // runs where the knots of all modes lie closer than kPanelMinBins bins on average
+  if (__reduce_add_sync(0xffffffffu, mine ? kk.y - kk.x : 0) * kPanelMinBins > i1 - i0) {
+    const double ts = __ldg(A.t_start + b), te = __ldg(A.t_end + b);
+    const double* xr = A.x + ((long long)b * M + (mine ? lane : 0)) * L;
+    const double lo = __ldg(xr), hi = __ldg(xr + L - 1);
+    const float per = (float)(L - 1) / logf((float)(hi / lo));
+    if (mine) {
+      PS.lo[lane] = lo;
+      PS.hi[lane] = hi;
+      PS.per[lane] = per;
+    }
+    __syncwarp();
+    for (;;) {
+      float dens = 0.0f;
+      if (mine && k >= 0 && k < L - 1) dens = (float)(df / (__ldg(xr + k + 1) - __ldg(xr + k)));
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) dens += __shfl_xor_sync(0xffffffffu, dens, o);
-    dens = __shfl_sync(0xffffffffu, dens, 0);
-    if (!(dens * (float)kPanelMinBins > 1.0f)) break;
-    const int n = min(kPanelDirect, i1 - i);
-    panel_scatter(A, PS, b, i, n, lane, k0, df, ts, te, dr, di, hh);
-    i += n;
-    if (i >= i1) return;
-    if (mine) k = segment_guess(xr, L, lo, hi, per, __dmul_rn(k0 + (double)i, df));
+      for (int o = 4; o > 0; o >>= 1) dens += __shfl_xor_sync(0xffffffffu, dens, o);
+      dens = __shfl_sync(0xffffffffu, dens, 0);
+      if (!(dens * (float)kPanelMinBins > 1.0f)) break;
+      const int n = min(kPanelDirect, i1 - i);
+      panel_scatter(A, PS, b, i, n, lane, k0, df, ts, te, dr, di, hh);
+      i += n;
+      if (i >= i1) return;
+      if (mine) k = segment_guess(xr, L, lo, hi, per, __dmul_rn(k0 + (double)i, df));
+    }
   }
-  if (mine && k < 0) next = first_bin_at(lo, k0, df, A.N);
+  // segment seg of mode m and the knot after it: this lane's element (quantity lane / 4,
+  // coefficient lane mod 4), lanes 0..3 also element 32 + lane of the ninth quantity
+  auto fetch = [&](int m, int seg) {
+    double* dst = PS.co[m][seg & (kPanelRing - 1)];
+    const long long o = ((long long)b * M + m) * L + seg;
+    const int cc = lane & 3;
+    const double* src = ((cc == 0) ? A.y : (cc == 1) ? A.c1 : (cc == 2) ? A.c2 : A.c3) + o;
+    copy8_async(dst + lane, src + (lane >> 2) * A.qstride);
+    if (lane < 4) copy8_async(dst + 32 + lane, src + 8 * A.qstride);
+    if (lane == 4) copy8_async(&PS.x[m][(seg + 1) & 7], A.x + o + 1);
+  };
+  for (int m = 0; m < M; ++m) {
+    const int ks = max(__shfl_sync(0xffffffffu, k, m), 0);
+    const int kz = min(__shfl_sync(0xffffffffu, klast, m), ks + kPanelRing - 1);
+    if (lane == 5 && ks <= kz) copy8_async(&PS.x[m][ks & 7], A.x + ((long long)b * M + m) * L + ks);
+    for (int s = ks; s <= kz; ++s) fetch(m, s);
+  }
+  copy_commit();
+  copy_wait<0>();
+  __syncwarp();
+  // per-lane state of mode `lane`: segment k, first bin of the next one, gate (2: nothing to add)
+  int next = 0, gate = 2;
+  auto enter = [&]() {  // lane's mode has arrived in segment k
+    gate = 2;
+    if (k < L - 1) {
+      const double x1 = PS.x[lane][(k + 1) & 7];
+      const double inv_df = 1.0 / df;
+      const double xb1 = fma(x1, inv_df, -k0);
+      next = first_bin_at(x1, xb1, k0, df, A.N);
+      if (k >= 0) {
+        const double* c = PS.co[lane][k & (kPanelRing - 1)];
+        const double x0 = PS.x[lane][k & 7];
+        gate = hull_gate(c + 8, x1 - x0, __ldg(A.t_start + b), __ldg(A.t_end + b));
+        PS.kb[lane] = fma(x0, inv_df, -k0);
+        PS.sl[lane] = make_float4((float)(c[5] * df), (float)(2.0 * c[6] * df * df),
+                                  (float)(3.0 * c[7] * df * df * df), 0.0f);
+        PS.xk[lane] = x0;
+      }
+    }
+    PS.slot[lane] = (gate != 2) ? (k & (kPanelRing - 1)) : -1;
+  };
+  if (mine) {
+    if (k < 0) {  // before the mode's first knot: wait for it
+      next = i1;
+      if (klast >= 0) {
+        const double x0 = PS.x[lane][0];
+        next = first_bin_at(x0, x0 / df - k0, k0, df, A.N);
+      }
+      PS.slot[lane] = -1;
+    } else {
+      enter();
+    }
+  }
   int cap = kPanelBins;  // longest panel that converged of late
-  double cb = 0.0, er = 1.0, ei = 0.0, Rr = 1.0, Ri = 0.0;  // carrier slope, e^{i b lane}, e^{32 i b}
-  bool fresh = true;  // windows still to be staged
+  float cb = 0.0f;  // carrier slope
+  double Rr = 1.0, Ri = 0.0;  // e^{32 i b}
+  PS.E[lane] = make_double2(1.0, 0.0);
   while (i < i1) {
-    // modes whose next knot lies at or before bin i move on; windows they left are staged
-    bool move = mine && k < L - 1 && next <= i && !(fresh && k >= 0);
-    while (__any_sync(0xffffffffu, move || fresh)) {
-      if (move) ++k;
-      if (!fresh) cap = min(2 * cap, kPanelBins);
-      const bool in = mine && k >= 0 && k < L - 1;
-      unsigned need = __ballot_sync(0xffffffffu, in && (k < klo || k >= klo + nst));
-      const unsigned staged = need;
-      while (need) {
-        const int m = __ffs(need) - 1;
-        need &= need - 1;
-        const int ks = __shfl_sync(0xffffffffu, k, m);
-        const int ns = min(NSEG, L - 1 - ks);
-        if (lane == m) {
-          klo = ks;
-          nst = ns;
-        }
-        stage_segments(A, S, b, m, ks, ns, lane);
+    // modes whose next knot lies at or before bin i move on
+    unsigned move = __ballot_sync(0xffffffffu, mine && k < L - 1 && next <= i);
+    while (move) {
+      cap = min(2 * cap, kPanelBins);
+      const bool go = (move >> lane) & 1u;
+      for (unsigned t = move; t; t &= t - 1) {
+        const int m = __ffs(t) - 1;
+        const int left = __shfl_sync(0xffffffffu, k, m);
+        const int last = __shfl_sync(0xffffffffu, klast, m);
+        if (left >= 0 && left + kPanelRing <= last) fetch(m, left + kPanelRing);
       }
+      copy_commit();
+      copy_wait<2>();  // the segment entered was asked for at least three groups ago
       __syncwarp();
-      if (staged) {  // whole-segment t(f) gates of the new windows
-        const int m = lane >> 2, sg = lane & 3;
-        static_assert(NSEG == 4 && FD_MAXM <= 8, "lanes = mode x staged segment");
-        const int ns = __shfl_sync(0xffffffffu, nst, m);
-        if (((staged >> m) & 1u) && sg < ns)
-          S.gate[m][sg] = segment_gate(&S.pc[m][sg][1][0], S.x[m][sg + 1] - S.x[m][sg], ts, te);
-        __syncwarp();
+      if (go) {
+        ++k;
+        enter();
       }
-      if (in && (move || fresh)) next = first_bin_at(S.x[lane][k + 1 - klo], k0, df, A.N);
-      fresh = false;
-      move = mine && k < L - 1 && next <= i;
+      move = __ballot_sync(0xffffffffu, go && k < L - 1 && next <= i);
     }
+    __syncwarp();
     // bins up to the next knot of any mode; the modes' phase slopes (rad per bin) at both ends
-    const bool in = mine && k >= 0 && k < L - 1;
-    const int gate = in ? S.gate[lane][k - klo] : 2;
-    int e = (mine && k < L - 1) ? next : i1;
-    e = __reduce_min_sync(0xffffffffu, e);
+    int e = __reduce_min_sync(0xffffffffu, (mine && k < L - 1) ? next : i1);
     e = min(min(e, i1), i + cap);
-    if (mine) PS.kl[lane] = (gate != 2) ? k - klo : -1;
-    double mx = -INFINITY, mn = INFINITY, cv = 0.0;
-    if (gate != 2) {
-      const double* c = &S.pc[lane][k - klo][0][0];
-      const double c1 = c[1], c2 = 2.0 * c[2], c3 = 3.0 * c[3], xk = S.x[lane][k - klo];
-      const double ua = __dmul_rn(k0 + (double)i, df) - xk;
-      const double uz = __dmul_rn(k0 + (double)(e - 1), df) - xk;
-      const double sa = fma(fma(c3, ua, c2), ua, c1) * df;
-      const double sz = fma(fma(c3, uz, c2), uz, c1) * df;
-      mx = fmax(sa, sz);
-      mn = fmin(sa, sz);
-      cv = mx - mn;
-    }
-    const unsigned act = __ballot_sync(0xffffffffu, gate != 2);
-    const unsigned edge = __ballot_sync(0xffffffffu, gate == 0);
     int n = e - i;
+    const unsigned act = __ballot_sync(0xffffffffu, gate != 2);
     if (act == 0u) {
       i = e;
       continue;
     }
-    __syncwarp();
-    if (edge) {
-      panel_direct(A, S, PS, i, n, lane, k0, df, ts, te, dr, di, hh);
-      __syncwarp();
+    if (__any_sync(0xffffffffu, gate == 0)) {
+      panel_direct<1, true>(A, PS, b, i, n, lane, k0, df, dr, di, hh);
       i = e;
       continue;
     }
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-      mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-      cv = fmax(cv, __shfl_xor_sync(0xffffffffu, cv, o));
+    float mx = -INFINITY, mn = INFINITY, cv = 0.0f;
+    if (gate != 2) {
+      const float4 a = PS.sl[lane];
+      const float ta = (float)((double)i - PS.kb[lane]), tz = ta + (float)(n - 1);
+      const float sa = fmaf(fmaf(a.z, ta, a.y), ta, a.x), sz = fmaf(fmaf(a.z, tz, a.y), tz, a.x);
+      mx = fmaxf(sa, sz);
+      mn = fminf(sa, sz);
+      cv = mx - mn;
     }
-    cv = __shfl_sync(0xffffffffu, cv, 0);
-    mx = __shfl_sync(0xffffffffu, mx, 0);
-    mn = __shfl_sync(0xffffffffu, mn, 0);
+    mx = order_value(__reduce_max_sync(0xffffffffu, order_key(mx)));
+    mn = order_value(__reduce_min_sync(0xffffffffu, order_key(mn)));
+    cv = order_value(__reduce_max_sync(0xffffffffu, order_key(cv)));
     // residual phase of the panel with a centred carrier: linear 0.25 (mx - mn) n, quadratic
     // cv n / 8 (a slope change of cv over n bins), both shrinking with n
-    const double lin = 0.25 * (mx - mn) * n, quad = 0.125 * cv * n;
+    const float lin = 0.25f * (mx - mn) * n, quad = 0.125f * cv * n;
     if (lin > kPanelDelta || quad > kPanelQuad) {
-      const double fit = n * fmin(1.0, fmin(kPanelDelta / lin, sqrt(kPanelQuad / quad)));
-      if (fit < kPanelMinBins) {
+      const float fit = n * fminf(1.0f, fminf(kPanelDelta / lin, sqrtf(kPanelQuad / quad)));
+      if (!(fit >= (float)kPanelMinBins)) {
         n = min(n, kPanelDirect);
-        panel_direct(A, S, PS, i, n, lane, k0, df, ts, te, dr, di, hh);
-        __syncwarp();
+        panel_direct<2, false>(A, PS, b, i, n, lane, k0, df, dr, di, hh);
         i += n;
         continue;
       }
-      const int pieces = (int)ceil((double)n / fit);
+      const int pieces = (int)ceilf((float)n / fit);
       n = min((n + pieces - 1) / pieces, (int)fit);
     }
-    if (!(0.5 * fmax(fabs(mx - cb), fabs(mn - cb)) * n <= kPanelDelta)) {
-      cb = 0.5 * (mx + mn);
-      sincos_cw(cb * (double)lane, &ei, &er);
-      sincos_cw(32.0 * cb, &Ri, &Rr);
+    if (!(0.5f * fmaxf(fabsf(mx - cb), fabsf(mn - cb)) * n <= kPanelDelta)) {
+      cb = 0.5f * (mx + mn);
+      double er, ei;
+      sincos_cw((double)cb * (double)lane, &ei, &er);
+      PS.E[lane] = make_double2(er, ei);
+      sincos_cw(32.0 * (double)cb, &Ri, &Rr);
     }
     double center, half;
     bool smooth;
     for (;;) {
       center = 0.5 * (double)(n - 1);
       half = fmax(center, 0.5);
-      panel_nodes(S, PS, M, lane, k0 + (double)i, center, half, df, cb, tau, row);
+      panel_nodes(PS, M, lane, k0 + (double)i, center, half, df, (double)cb);
       smooth = panel_smooth(PS, lane);
       if (smooth || n <= kPanelMinBins) break;
       n >>= 1;
       cap = n;
     }
     if (!smooth) {
-      panel_direct(A, S, PS, i, n, lane, k0, df, ts, te, dr, di, hh);
-      __syncwarp();
+      panel_direct<2, false>(A, PS, b, i, n, lane, k0, df, dr, di, hh);
       i += n;
       continue;
     }
     double zr, zi;
     panel_bins(A, PS, i, n, center, 1.0 / half, lane, Rr, Ri, zr, zi, hh);
-    dr = fma(zr, er, fma(-zi, ei, dr));
-    di -= fma(zr, ei, zi * er);
-    __syncwarp();
+    const double2 E = PS.E[lane];
+    dr = fma(zr, E.x, fma(-zi, E.y, dr));
+    di -= fma(zr, E.y, zi * E.x);
     i += n;
   }
+  copy_wait<0>();
+  __syncwarp();
 }
 
 }  // namespace bbhx

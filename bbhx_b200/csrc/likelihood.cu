@@ -249,7 +249,7 @@ struct FusedArgs {
   // written at gh[3 (gh_off[b] + i - sup_start[b]) + channel]; null in the likelihood calls
   cplx* gh;
   const long long* gh_off;
-  // uniform-grid record of data_freqs (k_grid_detect) enabling the phase recurrence, or null
+  // uniform-grid record of data_freqs (k_grid_detect), or null: panels / phase recurrence
   const struct GridInfo* grid;
   // work-queue counter, zero at launch: warps claim (tile, binary) items from it in increasing
   // order (claim_item)
@@ -259,8 +259,8 @@ struct FusedArgs {
 // Data grid of the form f_i = fl((k0 + i) df): numpy's k * df and rfftfreq grids, the form
 // BBHx's data streams take.  k_grid_detect verifies the form bit-exactly on the device for
 // three candidates of df (the rounded f[N-1] / (k0 + N - 1) and its two neighbours); bit c of
-// ok says candidate c reproduces every f_i.  The fused kernel then knows every bin's exact
-// frequency k df (as p + pe, an error-free product), which the phase recurrence needs.
+// ok says candidate c reproduces every f_i.  The kernels then know every bin's exact frequency
+// k df (as p + pe, an error-free product), which panels and phase recurrence need.
 struct GridInfo {
   double k0;
   double df[3];
@@ -477,7 +477,8 @@ struct alignas(16) WarpStage {
   int kst[FD_MAXM];
   int nst[FD_MAXM];
   int gate[FD_MAXM][NSEG];  // t(f) gate over the whole segment: 0 mixed, 1 all in, 2 all out
-  signed char cseg[FD_MAXCHUNK][FD_MAXM];  // staged segment holding a whole 128-bin chunk, or -1
+  // staged segment holding a whole 128-bin chunk, or -1 (FP64 single-problem tiles: 2 FD_TILE)
+  signed char cseg[2 * FD_MAXCHUNK][FD_MAXM];
 };
 
 // ---------------------------------------------------------------- phase recurrence
@@ -877,17 +878,17 @@ namespace bbhx {
 // functions, sin/cos of the reduced phase and the mode sum (the template) in FP32; the per-bin
 // products with data and weights in FP64 when the FP32 copies of data and weights are given
 // (the path of Likelihood and UnevenBatch), in FP32 without them.
-// GH (FP64 form only): also write d lnL / d h of every support bin to A.gh (gradient chain).
-// REC (FP64 form): the phase recurrence in the one-segment chunk path when the data grid is
-// uniform (A.grid), with its state in RS.
-template <bool MIXED, typename R, bool GH = false, bool REC = false>
+// GH (FP64 form only): also write d lnL / d h of every support bin to A.gh (gradient chain), with
+// the phase recurrence (state in RS) in the one-segment chunk path on uniform grids (A.grid).
+// PANEL (FP64 form): uniform grids go to panel_item, with its shared memory in PS.
+template <bool MIXED, typename R, bool GH = false, bool PANEL = false>
 __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, WarpStage<R>& S,
                                            RecStage* RS, PanelStage* PS, int lane) {
   const long long BML = A.qstride;
   const int L = A.L;
   bool uni = false;
   double gk0 = 0.0, gdf = 0.0;
-  if (!MIXED && A.grid != nullptr) {
+  if ((GH || PANEL) && A.grid != nullptr) {
     const unsigned ok = A.grid->ok & 7u;
     if (ok) {
       uni = true;
@@ -909,11 +910,11 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
       }
       return;
     }
-    if constexpr (!MIXED && !GH) {
+    if constexpr (PANEL) {
       if (uni) {
-        const int kk = (lane < A.M) ? A.segtab[q * A.M + lane].x : 0;
+        const int2 kk = (lane < A.M) ? A.segtab[q * A.M + lane] : make_int2(0, 0);
         double dr = 0.0, di = 0.0, hh = 0.0;
-        panel_item(A, S, *PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, gk0, gdf, dr, di, hh);
+        panel_item(A, *PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, gk0, gdf, dr, di, hh);
         for (int o = 16; o > 0; o >>= 1) {
           dr += __shfl_xor_sync(0xffffffffu, dr, o);
           di += __shfl_xor_sync(0xffffffffu, di, o);
@@ -930,7 +931,7 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
       }
     }
     // ---- stage this tile's segments for every mode
-    if (REC && lane < FD_MAXM) RS->next_chunk[lane] = -1;
+    if (GH && lane < FD_MAXM) RS->next_chunk[lane] = -1;
     if (lane < A.M) {
       const int2 kk = A.segtab[q * A.M + lane];
       const int klo = max(kk.x, 0), khi = min(kk.y, L - 2);
@@ -1016,7 +1017,7 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
           if (ka >= 0) {
             const int gate = S.gate[m][ka];
             if (gate == 2) continue;
-            if (REC && uni) {
+            if (GH && uni) {
               rec_chunk_mode(S, RS, m, ka, S.klo[m] + ka, gate, ck, c0, lane, fbin, ts, te, acc,
                              gk0, gdf, hstep);
               continue;
@@ -1143,7 +1144,7 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
               if (ka == kz) {  // one segment holds every bin of the chunk
                 const int gate = S.gate[m][kl0];
                 if (gate != 2) {
-                  if (REC && uni) {
+                  if (GH && uni) {
                     rec_chunk_mode(S, RS, m, kl0, klo, gate, ck, c0, lane, fbin, ts, te, acc, gk0,
                                    gdf, hstep);
                   } else {
@@ -1271,8 +1272,8 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
 template <bool MIXED, bool GH = false>
 constexpr size_t fused_smem_bytes() {
   using R = typename std::conditional<MIXED, float, double>::type;
-  return FD_WARPS * (sizeof(WarpStage<R>) +
-                     (MIXED ? 0 : GH ? sizeof(RecStage) : sizeof(PanelStage)));
+  constexpr size_t stage = sizeof(WarpStage<R>) + (GH ? sizeof(RecStage) : 0);
+  return FD_WARPS * (MIXED || stage > sizeof(PanelStage) ? stage : sizeof(PanelStage));
 }
 
 template <bool MIXED, bool GH = false>
@@ -1283,12 +1284,48 @@ __global__ void __launch_bounds__(FD_WARPS * 32, MIXED ? 4 : 3) k_direct_fused(F
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   WarpStage<R>& S = reinterpret_cast<WarpStage<R>*>(smem_raw)[warp];
-  unsigned char* extra = smem_raw + FD_WARPS * sizeof(WarpStage<R>);
-  RecStage* RS = reinterpret_cast<RecStage*>(extra) + warp;
-  PanelStage* PS = reinterpret_cast<PanelStage*>(extra) + warp;
+  RecStage* RS = reinterpret_cast<RecStage*>(smem_raw + FD_WARPS * sizeof(WarpStage<R>)) + warp;
+  if (!MIXED && !GH && (A.grid->ok & 7u)) return;  // k_direct_panel's
   const long long nitems = (long long)A.ntiles * A.B;
   for (long long q = claim_item(A.next, lane); q < nitems; q = claim_item(A.next, lane))
-    fused_item<MIXED, R, GH, GH>(A, q, S, RS, PS, lane);
+    fused_item<MIXED, R, GH>(A, q, S, RS, nullptr, lane);
+}
+
+// FP64 form on uniform grids (panel_item); returns at once on others, which k_direct_fused takes.
+__global__ void __launch_bounds__(FD_WARPS * 32, 3) k_direct_panel(FusedArgs A) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const unsigned ok = A.grid->ok & 7u;
+  if (ok == 0u) return;
+  const int lane = threadIdx.x & 31;
+  PanelStage& PS = reinterpret_cast<PanelStage*>(smem_raw)[threadIdx.x >> 5];
+  const double k0 = A.grid->k0, df = A.grid->df[(ok & 1u) ? 0 : (ok & 2u) ? 1 : 2];
+  const long long nitems = (long long)A.ntiles * A.B;
+  long long nxt = claim_item(A.next, lane);
+  while (nxt < nitems) {
+    const long long q = nxt;
+    nxt = claim_item(A.next, lane);  // the next item's number arrives while this one is summed
+    const int tile = (int)(q / A.B);
+    const int b = (int)(q - (long long)tile * A.B);
+    const int s0 = __ldg(A.sup_start + b), s1 = s0 + __ldg(A.sup_len + b);
+    const int t0 = tile * A.tile;
+    double dr = 0.0, di = 0.0, hh = 0.0;
+    if (t0 < s1 && t0 + A.tile > s0) {
+      const int2 kk = (lane < A.M) ? A.segtab[q * A.M + lane] : make_int2(0, 0);
+      panel_item(A, PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, k0, df, dr, di, hh);
+      for (int o = 16; o > 0; o >>= 1) {
+        dr += __shfl_xor_sync(0xffffffffu, dr, o);
+        di += __shfl_xor_sync(0xffffffffu, di, o);
+        hh += __shfl_xor_sync(0xffffffffu, hh, o);
+      }
+    }
+    if (lane == 0) {
+      double* P = A.partials + 3 * q;
+      P[0] = dr;
+      P[1] = di;
+      P[2] = hh;
+    }
+    __syncwarp();
+  }
 }
 
 // Several independent problems (groups: own data stream, grid length L, mode count M,
@@ -1369,7 +1406,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32, (MIXED && !HET) ? 4 : 3)
   const int warp = threadIdx.x >> 5;
   unsigned char* mine = smem_raw + (size_t)warp * slot;
   WarpStage<R>& S = *reinterpret_cast<WarpStage<R>*>(mine);
-  PanelStage* PS = reinterpret_cast<PanelStage*>(mine + sizeof(WarpStage<R>));
+  PanelStage* PS = reinterpret_cast<PanelStage*>(mine);
   const long long nh = HM->woff[HM->ngroups];
   const long long total = nh + MA->off[MA->ngroups];
   int g = -1, hg = -1;
@@ -1399,7 +1436,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32, (MIXED && !HET) ? 4 : 3)
         for (int i = lane; i < n8; i += 32) dst[i] = src[i];
         __syncwarp();
       }
-      fused_item<MIXED, R>(gcur[warp], qd - MA->off[g], S, nullptr, PS, lane);
+      fused_item<MIXED, R, false, !MIXED>(gcur[warp], qd - MA->off[g], S, nullptr, PS, lane);
     }
   }
 }
@@ -1502,12 +1539,12 @@ unsigned resident_grid(K kernel, size_t smem, long long nitems) {
   return (unsigned)std::max<long long>(1, std::min<long long>(want, (long long)per_sm * sm_count()));
 }
 
-// Data bins per work item of a single-problem launch: the largest tile that still gives every
-// resident warp several items, since an item of a low-frequency tile takes many times the
-// average (few binaries: the call ends when its slowest item does).
-inline int fused_tile(int N, int B) {
+// Data bins per work item of a single-problem launch: the largest tile up to `tile` that still
+// gives every resident warp several items, since an item of a low-frequency tile takes many times
+// the average and the call ends when its slowest item does (B = 1, 1 yr: 1.03 ms at 4096 bins,
+// 0.25 ms at 512; B = 1024: 1.1 ms less at 8192 bins than at 4096).
+inline int fused_tile(int N, int B, int tile) {
   const long long warps = (long long)sm_count() * 3 * FD_WARPS;
-  int tile = FD_TILE;
   while (tile > 256 && ((long long)N + tile - 1) / tile * B < 8 * warps) tile >>= 1;
   return tile;
 }
@@ -1980,7 +2017,7 @@ int bbhx_direct_like_fused(double* d_h, double* h_h, const double* data_freqs, c
   BBHX_REQUIRE(num_modes <= FD_MAXM, "num_modes must be <= 6");
   if (num_bin_all == 0) return OK;
   cudaStream_t s = (cudaStream_t)stream;
-  const int tile = fused_tile(data_length, num_bin_all);
+  const int tile = fused_tile(data_length, num_bin_all, precision == 1 ? FD_TILE : 2 * FD_TILE);
   const int ntiles = (data_length + tile - 1) / tile;
   const long long nitems = (long long)ntiles * num_bin_all;
   int* sup = nullptr;
@@ -2042,12 +2079,16 @@ int bbhx_direct_like_fused(double* d_h, double* h_h, const double* data_freqs, c
       if (!r) kernel<<<resident_grid(kernel, sm, nitems), FD_WARPS * 32, sm, s>>>(A);
       return r;
     };
-    if (!st)
-      st = (precision == 1)
-               ? launch(k_direct_fused<true>, fused_smem_bytes<true>(),
-                        "cudaFuncSetAttribute(k_direct_fused<true>)")
-               : launch(k_direct_fused<false>, fused_smem_bytes<false>(),
-                        "cudaFuncSetAttribute(k_direct_fused<false>)");
+    if (!st && precision == 1)
+      st = launch(k_direct_fused<true>, fused_smem_bytes<true>(),
+                  "cudaFuncSetAttribute(k_direct_fused<true>)");
+    if (!st && precision == 0) {  // one of the two does the work, by the grid record
+      st = launch(k_direct_panel, FD_WARPS * sizeof(PanelStage), "cudaFuncSetAttribute(k_direct_panel)");
+      if (!st) st = launch_status("k_direct_panel");
+      if (!st)
+        st = launch(k_direct_fused<false>, fused_smem_bytes<false>(),
+                    "cudaFuncSetAttribute(k_direct_fused<false>)");
+    }
     if (!st) st = launch_status("k_direct_fused");
   }
   if (!st) {
