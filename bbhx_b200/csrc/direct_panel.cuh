@@ -122,22 +122,6 @@ __device__ __forceinline__ int segment_guess(const double* __restrict__ xr, int 
   return a - 1;
 }
 
-// t(f) gate over a whole segment from the control points of its cubic (their hull holds it): 1 all
-// inside the observation window, 2 all outside, 0 undecided (per-bin gate).
-__device__ __forceinline__ int hull_gate(const double* c, double h, double ts, double te) {
-  const double a = c[1] * h, q = c[2] * h * h;
-  const double p1 = c[0] + a * (1.0 / 3.0);
-  const double p2 = c[0] + (2.0 * a + q) * (1.0 / 3.0);
-  const double p3 = c[0] + a + q + c[3] * h * h * h;
-  const double lo = fmin(fmin(c[0], p1), fmin(p2, p3));
-  const double hi = fmax(fmax(c[0], p1), fmax(p2, p3));
-  const double eps = 1e-6;  // s: far above the rounding of t(f), as in segment_gate
-  if (!(lo == lo) || !(hi == hi)) return 0;
-  if (lo >= ts + eps && (te <= 0.0 || hi <= te - eps)) return 1;
-  if (hi < ts - eps || (te > 0.0 && lo > te + eps)) return 2;
-  return 0;
-}
-
 // Order-preserving integer of a float and back (warp max / min by integer reductions).
 __device__ __forceinline__ int order_key(float v) {
   const int b = __float_as_int(v);
@@ -312,8 +296,61 @@ __device__ __forceinline__ void panel_bins(const FusedArgs& A, const PanelStage&
   }
 }
 
-// One bin's template acc (6 reals) times weights and data, into the sums.
-__device__ __forceinline__ void bin_products(const FusedArgs& A, int i, const double* acc,
+template <bool GH>
+__device__ __forceinline__ void bin_products(const FusedArgs& A, cplx* gh, int i, const double* acc,
+                                             double& dr, double& di, double& hh);
+
+// panel_bins for the gradient: the same sums and d lnL / d h = 4 w (d~ - w h) of every bin, which
+// needs the carrier e^{i b (i - ia)} bin by bin (rotated along the lane's bins).
+__device__ __forceinline__ void panel_bins_gh(const FusedArgs& A, cplx* gh, const PanelStage& PS,
+                                              int ia, int n, double center, double inv_half,
+                                              int lane, double Rr, double Ri, double& dr,
+                                              double& di, double& hh) {
+  const double s0 = ((double)lane - center) * inv_half, ds = 32.0 * inv_half;
+  const double2 E = PS.E[lane];
+  double er = E.x, ei = E.y;
+  for (int i = lane, j = 0; i < n; i += 64, j += 2) {
+    double f[2][6], s[2], cr[2], ci[2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      s[t] = fma((double)(j + t), ds, s0);
+      cr[t] = er;
+      ci[t] = ei;
+      cmul_inplace(er, ei, Rr, Ri);
+    }
+#pragma unroll
+    for (int ch = 0; ch < 3; ++ch) {
+      double qr[2], qi[2];
+      const double2 top = PS.C[ch][kPanelNodes - 1];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        qr[t] = top.x;
+        qi[t] = top.y;
+      }
+#pragma unroll
+      for (int p = kPanelNodes - 2; p >= 0; --p) {
+        const double2 c = PS.C[ch][p];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          qr[t] = fma(qr[t], s[t], c.x);
+          qi[t] = fma(qi[t], s[t], c.y);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {  // h = conj(Q e^{i c})
+        f[t][2 * ch] = fma(qr[t], cr[t], -qi[t] * ci[t]);
+        f[t][2 * ch + 1] = -fma(qr[t], ci[t], qi[t] * cr[t]);
+      }
+    }
+    bin_products<true>(A, gh, ia + i, f[0], dr, di, hh);
+    if (i + 32 < n) bin_products<true>(A, gh, ia + i + 32, f[1], dr, di, hh);
+  }
+}
+
+// One bin's template acc (6 reals) times weights and data, into the sums; GH: and its d lnL / d h =
+// 4 w (d~ - w h) to gh[3 i + channel] (gh addressed by data bin).
+template <bool GH>
+__device__ __forceinline__ void bin_products(const FusedArgs& A, cplx* gh, int i, const double* acc,
                                              double& dr, double& di, double& hh) {
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
@@ -324,13 +361,15 @@ __device__ __forceinline__ void bin_products(const FusedArgs& A, int i, const do
     dr = fma(d.x, hr, fma(d.y, hi, dr));
     di = fma(d.x, hi, fma(-d.y, hr, di));
     hh = fma(hr, hr, fma(hi, hi, hh));
+    if (GH) gh[3LL * i + c] = mk(4.0 * w * (d.x - hr), 4.0 * w * (d.y - hi));
   }
 }
 
 // The n bins from ia one by one (lanes over bins) where the knots lie as close as the bins: every
 // bin finds its own segment of each mode and reads the spline arrays.
-__device__ __forceinline__ void panel_scatter(const FusedArgs& A, const PanelStage& PS, int b,
-                                              int ia, int n, int lane, double k0, double df,
+template <bool GH>
+__device__ __forceinline__ void panel_scatter(const FusedArgs& A, cplx* gh, const PanelStage& PS,
+                                              int b, int ia, int n, int lane, double k0, double df,
                                               double ts, double te, double& dr, double& di,
                                               double& hh) {
   for (int i = ia + lane; i < ia + n; i += 32) {
@@ -342,15 +381,15 @@ __device__ __forceinline__ void panel_scatter(const FusedArgs& A, const PanelSta
       if (k >= 0 && k < A.L - 1)
         accumulate_bin_src(GlobalCoef{A, o + k, __ldg(A.x + o + k)}, f, ts, te, acc);
     }
-    bin_products(A, i, acc, dr, di, hh);
+    bin_products<GH>(A, gh, i, acc, dr, di, hh);
   }
 }
 
 // The n bins from ia one by one, G bins per lane at a time: runs where a mode crosses the
 // observation window (GATE: its t(f) decides bin by bin) or the modes' phases do not stay
 // together.
-template <int G, bool GATE>
-__device__ __forceinline__ void panel_direct(const FusedArgs& A, const PanelStage& PS, int b,
+template <int G, bool GATE, bool GH>
+__device__ __forceinline__ void panel_direct(const FusedArgs& A, cplx* gh, const PanelStage& PS, int b,
                                              int ia, int n, int lane, double k0, double df,
                                              double& dr, double& di, double& hh) {
   double ts = 0.0, te = 0.0;
@@ -412,7 +451,7 @@ __device__ __forceinline__ void panel_direct(const FusedArgs& A, const PanelStag
     }
 #pragma unroll
     for (int j = 0; j < G; ++j)
-      if (i + 32 * j < n) bin_products(A, ia + i + 32 * j, acc[j], dr, di, hh);
+      if (i + 32 * j < n) bin_products<GH>(A, gh, ia + i + 32 * j, acc[j], dr, di, hh);
   }
   __syncwarp();
 }
@@ -420,11 +459,15 @@ __device__ __forceinline__ void panel_direct(const FusedArgs& A, const PanelStag
 // Bins [i0, i1) of binary b (inside its support) by one warp; kk = the segments of bins i0 and
 // i1 - 1 in lanes 0 .. M-1 (-1 before a mode's first knot, L-1 past its last).  Lane m walks mode
 // m.  When a mode enters segment k its freed ring slot is refilled with segment k + 3 by
-// asynchronous copies, three entries ahead of their use.  Per-lane partial sums into dr, di, hh.
+// asynchronous copies, three entries ahead of their use.  Per-lane partial sums into dr, di, hh;
+// GH: also d lnL / d h of every bin to A.gh (gradient chain).
+template <bool GH>
 __device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, int b, int i0,
                                            int i1, int2 kk, int lane, double k0, double df,
                                            double& dr, double& di, double& hh) {
   const int M = A.M, L = A.L;
+  cplx* gh = nullptr;
+  if (GH) gh = A.gh + 3 * (__ldg(A.gh_off + b) - (long long)__ldg(A.sup_start + b));
   const bool mine = lane < M;
   int k = mine ? kk.x : L - 1;
   const int klast = mine ? min(kk.y, L - 2) : -1;  // last segment of the item
@@ -449,7 +492,7 @@ __device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, i
       dens = __shfl_sync(0xffffffffu, dens, 0);
       if (!(dens * (float)kPanelMinBins > 1.0f)) break;
       const int n = min(kPanelDirect, i1 - i);
-      panel_scatter(A, PS, b, i, n, lane, k0, df, ts, te, dr, di, hh);
+      panel_scatter<GH>(A, gh, PS, b, i, n, lane, k0, df, ts, te, dr, di, hh);
       i += n;
       if (i >= i1) return;
       if (mine) k = segment_guess(xr, L, lo, hi, per, __dmul_rn(k0 + (double)i, df));
@@ -540,11 +583,12 @@ __device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, i
     int n = e - i;
     const unsigned act = __ballot_sync(0xffffffffu, gate != 2);
     if (act == 0u) {
+      if (GH) panel_direct<1, false, GH>(A, gh, PS, b, i, n, lane, k0, df, dr, di, hh);  // h = 0
       i = e;
       continue;
     }
     if (__any_sync(0xffffffffu, gate == 0)) {
-      panel_direct<1, true>(A, PS, b, i, n, lane, k0, df, dr, di, hh);
+      panel_direct<1, true, GH>(A, gh, PS, b, i, n, lane, k0, df, dr, di, hh);
       i = e;
       continue;
     }
@@ -567,7 +611,7 @@ __device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, i
       const float fit = n * fminf(1.0f, fminf(kPanelDelta / lin, sqrtf(kPanelQuad / quad)));
       if (!(fit >= (float)kPanelMinBins)) {
         n = min(n, kPanelDirect);
-        panel_direct<2, false>(A, PS, b, i, n, lane, k0, df, dr, di, hh);
+        panel_direct<2, false, GH>(A, gh, PS, b, i, n, lane, k0, df, dr, di, hh);
         i += n;
         continue;
       }
@@ -593,15 +637,19 @@ __device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, i
       cap = n;
     }
     if (!smooth) {
-      panel_direct<2, false>(A, PS, b, i, n, lane, k0, df, dr, di, hh);
+      panel_direct<2, false, GH>(A, gh, PS, b, i, n, lane, k0, df, dr, di, hh);
       i += n;
       continue;
     }
-    double zr, zi;
-    panel_bins(A, PS, i, n, center, 1.0 / half, lane, Rr, Ri, zr, zi, hh);
-    const double2 E = PS.E[lane];
-    dr = fma(zr, E.x, fma(-zi, E.y, dr));
-    di -= fma(zr, E.y, zi * E.x);
+    if constexpr (GH) {
+      panel_bins_gh(A, gh, PS, i, n, center, 1.0 / half, lane, Rr, Ri, dr, di, hh);
+    } else {
+      double zr, zi;
+      panel_bins(A, PS, i, n, center, 1.0 / half, lane, Rr, Ri, zr, zi, hh);
+      const double2 E = PS.E[lane];
+      dr = fma(zr, E.x, fma(-zi, E.y, dr));
+      di -= fma(zr, E.y, zi * E.x);
+    }
     i += n;
   }
   copy_wait<0>();

@@ -24,6 +24,7 @@
 #include "capi_internal.cuh"
 #include "frames.cuh"
 #include "gradient_model.cuh"
+#include "spline_eval.cuh"
 #include "tridiag.cuh"
 
 namespace bbhx {
@@ -120,7 +121,7 @@ k_adj_coeffs(double* ybd, double* cb1, double* cb2, double* cb3, const cplx* gh,
              const long long* off, const int* start, const int* len, SplineRefs S,
              const double* data_freqs, int N, const double* t_start, const double* t_end, int b0,
              int nb, unsigned long long* next) {
-  __shared__ double scw[ADJ_THREADS / 32][36];  // the segment's (y, c1, c2, c3) x 9
+  __shared__ __align__(16) double scw[ADJ_THREADS / 32][36];  // the segment's (y, c1, c2, c3) x 9
   const int lane = threadIdx.x & 31;
   double* cw = scw[threadIdx.x >> 5];
   const int mp = lane >> 2, mk = lane & 3;
@@ -149,37 +150,70 @@ k_adj_coeffs(double* ybd, double* cb1, double* cb2, double* cb3, const cplx* gh,
 #pragma unroll
     for (int i = 0; i < 32; ++i) mom[i] = 0.0;
     const double xk = xs[s];
-    for (int k = k0 + lane; k < k1; k += 32) {
-      const double u = data_freqs[k] - xk;
-      double q[9];
+    // the whole segment against the observation window: t(f) is evaluated only where it decides
+    const int gate = hull_gate(cw + 8, xs[s + 1] - xk, ts, te);
+    auto coef = [&](int p, double* c) {
+      const double2 lo = *reinterpret_cast<const double2*>(cw + 4 * p);
+      const double2 hi = *reinterpret_cast<const double2*>(cw + 4 * p + 2);
+      c[0] = lo.x; c[1] = lo.y; c[2] = hi.x; c[3] = hi.y;
+    };
+    auto cubic = [](const double* c, double u) { return c[0] + u * (c[1] + u * (c[2] + u * c[3])); };
+    // two bins per lane share every coefficient read
+    for (int k = k0 + lane; k < k1 && gate != 2; k += 64) {
+      double u[2], cs[2], sn[2], am[2], a0[2], a1[2], v[2][6], c[4], e[4];
+      bool in[2];
+      coef(1, c);
 #pragma unroll
-      for (int p = 0; p < 9; ++p)
-        q[p] = cw[4 * p] + u * (cw[4 * p + 1] + u * (cw[4 * p + 2] + u * cw[4 * p + 3]));
-      if (!tf_gate(q[2], ts, te)) continue;
-      const cplx* g = gh + (off[bl] + (k - st)) * 3;
-      double sn, cs;
-      sincos_cw(q[1], &sn, &cs);
-      const double er = cs, ei = sn;                  // e^{i phase}
-      const double aer = q[0] * er, aei = q[0] * ei;  // A e^{i phase}
-      double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      for (int j = 0; j < 2; ++j) {
+        in[j] = k + 32 * j < k1;
+        const int kj = in[j] ? k + 32 * j : k;
+        u[j] = data_freqs[kj] - xk;
+        sincos_cw(cubic(c, u[j]), &sn[j], &cs[j]);
+        const double2* g = reinterpret_cast<const double2*>(gh + (off[bl] + (kj - st)) * 3);
+#pragma unroll
+        for (int ch = 0; ch < 3; ++ch) {  // V = g e^{i phase}
+          const double2 w = __ldg(g + ch);
+          v[j][2 * ch] = w.x * cs[j] - w.y * sn[j];
+          v[j][2 * ch + 1] = w.x * sn[j] + w.y * cs[j];
+        }
+      }
+      if (gate == 0) {
+        coef(2, c);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) in[j] = in[j] && tf_gate(cubic(c, u[j]), ts, te);
+      }
+      coef(0, c);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        am[j] = cubic(c, u[j]);
+        a0[j] = a1[j] = 0.0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) v[j][q] = in[j] ? v[j][q] : 0.0;
+      }
+      // dL = Re(V d(T A)): d / dA = Re(V T), d / dphase = -A Im(V T), d / dT = A V
 #pragma unroll
       for (int ch = 0; ch < 3; ++ch) {
-        const cplx u_ = g[ch];
-        const double tr = q[3 + 2 * ch], ti = q[4 + 2 * ch];
-        // dL = Re(u dW), W = T A e^{i phase}
-        const double wr = tr * aer - ti * aei, wi = tr * aei + ti * aer;
-        a[0] += u_.re * (tr * er - ti * ei) - u_.im * (tr * ei + ti * er);
-        a[1] += -(u_.re * wi + u_.im * wr);
-        a[2 + 2 * ch] = u_.re * aer - u_.im * aei;
-        a[3 + 2 * ch] = -(u_.re * aei + u_.im * aer);
-      }
-      const double u2 = u * u, u3 = u2 * u;
+        coef(3 + 2 * ch, c);
+        coef(4 + 2 * ch, e);
 #pragma unroll
-      for (int p = 0; p < 8; ++p) {
-        mom[4 * p] += a[p];
-        mom[4 * p + 1] = fma(a[p], u, mom[4 * p + 1]);
-        mom[4 * p + 2] = fma(a[p], u2, mom[4 * p + 2]);
-        mom[4 * p + 3] = fma(a[p], u3, mom[4 * p + 3]);
+        for (int j = 0; j < 2; ++j) {
+          const double tr = cubic(c, u[j]), ti = cubic(e, u[j]);
+          a0[j] += tr * v[j][2 * ch] - ti * v[j][2 * ch + 1];
+          a1[j] += tr * v[j][2 * ch + 1] + ti * v[j][2 * ch];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const double u2 = u[j] * u[j], u3 = u2 * u[j];
+#pragma unroll
+        for (int p = 0; p < 8; ++p) {
+          const double a = (p == 0) ? a0[j] : (p == 1) ? -am[j] * a1[j]
+                           : (p & 1) ? -am[j] * v[j][p - 2] : am[j] * v[j][p - 2];
+          mom[4 * p] += a;
+          mom[4 * p + 1] = fma(a, u[j], mom[4 * p + 1]);
+          mom[4 * p + 2] = fma(a, u2, mom[4 * p + 2]);
+          mom[4 * p + 3] = fma(a, u3, mom[4 * p + 3]);
+        }
       }
     }
     const double acc = warp_transpose_sum32(mom, lane);
@@ -352,12 +386,16 @@ __global__ void k_spline_adj(double* ybar, double* xbar, const double* ybd, cons
 // point's own frequency; To moves with lam and beta.  One thread per (local binary, mode)
 // repeats the forward's crossing search on the forward's default grid f0 and its t(f) tf0
 // ([B, M, L] each), evaluates the straddling points as duals and writes
-// wreg[row][0][k] = d flo / flo and wreg[row][1][k] = d fhi / fhi for the pass's directions.
+// wreg[pass][row][0][k] = d flo / flo and wreg[pass][row][1][k] = d fhi / fhi for the directions of
+// pass blockIdx.y.
 __global__ void k_regrid_tangents(double* wreg, const ModeCoeffsT<GD>* coeffs, const double* P,
                                   int B, int b0, int nb, int M, int L, const double* f0,
                                   const double* tf0, const double* t_start, const double* t_end,
-                                  double tL_start, double tL_end, int k0) {
+                                  double tL_start, double tL_end) {
   const long long n = (long long)nb * M;
+  const int k0 = blockIdx.y * GRAD_CHUNK;
+  coeffs += blockIdx.y * n;
+  wreg += blockIdx.y * n * 2 * GRAD_CHUNK;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     const int bl = (int)(t / M), m = (int)(t % M);
@@ -431,7 +469,8 @@ using namespace bbhx;
 
 namespace {
 constexpr long long kGhBudget = 1ll << 29;  // complex entries of d lnL / d h per batch (8 GB)
-constexpr int kDirectGradChunk = 512;
+constexpr int kDirectGradChunk = 512;  // binaries per batch of d lnL / d h
+constexpr int kDirectGradSub = 128;    // and per set of dual-number records (all passes at once)
 }  // namespace
 
 extern "C" {
@@ -479,16 +518,19 @@ int bbhx_direct_like_grad(void* orbits, void* d_h, void* h_h, double* grad, cons
   // adjoint arrays over all binaries, dual records and d lnL / d h per batch
   const size_t nall = (size_t)9 * B * M * L;
   const bool moving = f_default != nullptr && tf_default != nullptr;
-  double *ybd = nullptr, *cb = nullptr, *ybar = nullptr, *xbar = nullptr, *wreg = nullptr;
+  double *ybd = nullptr, *cb = nullptr, *ybar = nullptr, *xbar = nullptr, *wreg = nullptr,
+         *gpart = nullptr;
   ModeCoeffsT<GD>* cD = nullptr;
   ResponseModeT<GD>* rD = nullptr;
   const int chunk = std::min(B, kDirectGradChunk);
+  const int sub = std::min(B, kDirectGradSub);  // binaries per record set-up, all passes
+  const size_t nrec = (size_t)sub * M * GRAD_PASSES;
   if (!st) {
-    const size_t nscratch = nall * 5 + (size_t)B * M * L + (size_t)chunk * M * 2 * GRAD_CHUNK;
+    const size_t nscratch = nall * 5 + (size_t)B * M * L + nrec * 3 * GRAD_CHUNK;
     // + one 8-byte word after the arrays: the work-queue counter of k_adj_coeffs
     if (pool_alloc((void**)&ybd, sizeof(double) * (nscratch + 1), s) != cudaSuccess ||
-        pool_alloc((void**)&cD, sizeof(ModeCoeffsT<GD>) * (size_t)chunk * M, s) != cudaSuccess ||
-        pool_alloc((void**)&rD, sizeof(ResponseModeT<GD>) * (size_t)chunk * M, s) != cudaSuccess) {
+        pool_alloc((void**)&cD, sizeof(ModeCoeffsT<GD>) * nrec, s) != cudaSuccess ||
+        pool_alloc((void**)&rD, sizeof(ResponseModeT<GD>) * nrec, s) != cudaSuccess) {
       set_error("device allocation of the gradient scratch failed");
       st = ERR_CUDA;
     }
@@ -498,9 +540,10 @@ int bbhx_direct_like_grad(void* orbits, void* d_h, void* h_h, double* grad, cons
     ybar = cb + 3 * nall;
     xbar = ybar + nall;
     wreg = xbar + (size_t)B * M * L;
+    gpart = wreg + nrec * 2 * GRAD_CHUNK;
     // ybd / cb rows not written by k_adj_coeffs stay zero; wreg is zero for fixed knots
     if (cudaMemsetAsync(ybd, 0, sizeof(double) * nall * 4, s) != cudaSuccess ||
-        cudaMemsetAsync(wreg, 0, sizeof(double) * (size_t)chunk * M * 2 * GRAD_CHUNK, s) != cudaSuccess) {
+        cudaMemsetAsync(wreg, 0, sizeof(double) * nrec * 2 * GRAD_CHUNK, s) != cudaSuccess) {
       set_error("cudaMemsetAsync failed");
       st = ERR_CUDA;
     }
@@ -541,7 +584,7 @@ int bbhx_direct_like_grad(void* orbits, void* d_h, void* h_h, double* grad, cons
     if (!st) {
       const long long warps = (long long)nb * M * (L - 1);
       unsigned long long* next = reinterpret_cast<unsigned long long*>(
-          ybd + nall * 5 + (size_t)B * M * L + (size_t)chunk * M * 2 * GRAD_CHUNK);
+          gpart + nrec * GRAD_CHUNK);
       st = cuda_status(cudaMemsetAsync(next, 0, sizeof(unsigned long long), s),
                        "work-queue counter");
       // resident CTAs only: every warp claims segments until the queue drains (a segment holds
@@ -567,23 +610,31 @@ int bbhx_direct_like_grad(void* orbits, void* d_h, void* h_h, double* grad, cons
           ybar, xbar, ybd, cb, cb + nall, cb + 2 * nall, S, b0, nb);
       st = launch_status("k_spline_adj");
     }
-    for (int k0 = 0; !st && k0 < NGRAD; k0 += GRAD_CHUNK) {
-      k_grad_setup<<<grid_for((long long)nb * M, 64), 64, 0, s>>>(cD, rD, params, B, b0, nb, ells,
-                                                                  mms, M, qnm_table, qnm_n, dspin,
-                                                                  run_phenomd, k0);
+    for (int c0 = 0; !st && c0 < nb; c0 += sub) {
+      const int b1 = b0 + c0, n1 = std::min(sub, nb - c0);
+      const dim3 rows(grid_for((long long)n1 * M, 64), GRAD_PASSES);
+      k_grad_setup<<<rows, 64, 0, s>>>(cD, rD, params, B, b1, n1, ells, mms, M, qnm_table, qnm_n,
+                                       dspin, run_phenomd);
       st = launch_status("k_grad_setup");
-      if (st) break;
-      if (moving) {
-        k_regrid_tangents<<<grid_for((long long)nb * M, 64), 64, 0, s>>>(
-            wreg, cD, params, B, b0, nb, M, L, f_default, tf_default, t_start, t_end,
-            t_obs_start_L, t_obs_end_L, k0);
+      if (!st && moving) {
+        k_regrid_tangents<<<rows, 64, 0, s>>>(wreg, cD, params, B, b1, n1, M, L, f_default,
+                                              tf_default, t_start, t_end, t_obs_start_L,
+                                              t_obs_end_L);
         st = launch_status("k_regrid_tangents");
-        if (st) break;
       }
-      k_contract_direct<<<(unsigned)std::min(nb, nsm * 8), 128, 0, s>>>(
-          grad, cD, rD, ((OrbitHandle*)orbits)->tab, params, B, b0, nb, t_init, x, ybar, xbar,
-          wreg, TDItag, rescaled, tdi2, M, L, k0);
-      st = launch_status("k_contract_direct");
+      if (!st) {
+        const int mg = contract_modes(n1, M);
+        k_contract_direct<<<dim3(contract_blocks(n1, M, mg), GRAD_PASSES), 128, 0, s>>>(
+            gpart, cD, rD, ((OrbitHandle*)orbits)->tab, params, B, b1, n1, t_init, x, ybar, xbar,
+            wreg, TDItag, rescaled, tdi2, M, L, mg);
+        st = launch_status("k_contract_direct");
+      }
+      if (!st) {
+        const int mg = contract_modes(n1, M);
+        k_grad_sum<<<grid_for((long long)n1 * NGRAD, 128), 128, 0, s>>>(grad, gpart, b1, n1,
+                                                                       (M + mg - 1) / mg);
+        st = launch_status("k_grad_sum");
+      }
     }
     if (gh) pool_free(gh, s);
     if (off) pool_free(off, s);

@@ -8,11 +8,17 @@
 //   5 phi_ref (5)   6 inc (7)   7 lam (8)   8 beta (9)   9 psi (10)   10 t_ref [s] (11)
 // f_ref (row 6) does not enter the model (the reference frequency is the amplitude peak).
 //
-// The 11 directions are carried GRAD_CHUNK at a time (passes k0 = 0, GRAD_CHUNK, ...): a
+// The 11 directions are carried GRAD_CHUNK at a time (pass p: directions p GRAD_CHUNK, ...): a
 // dual number of GRAD_CHUNK tangents keeps much more of the model's working set in registers
-// than one of 11 tangents, which spills to local memory.
+// than one of 11 tangents, which spills to local memory.  The passes are independent and run side
+// by side in one launch (blockIdx.y), each with its own records; with few binaries their modes are
+// spread over blocks too.  One block per binary and a launch per pass left the GPU mostly idle at
+// a few hundred binaries (set-up, knot tangents and contraction of 128 binaries: 2.4 -> 0.5 ms).
 #pragma once
 
+#include <algorithm>
+
+#include "capi_internal.cuh"
 #include "bbhx_common.cuh"
 #include "dual.cuh"
 #include "phenomhm_model.cuh"
@@ -62,8 +68,11 @@ __device__ inline GradParams load_grad_params(const double* P, int B, int b, int
 static __global__ void k_grad_setup(ModeCoeffsT<GD>* coeffs, ResponseModeT<GD>* rmodes,
                                     const double* P, int B, int b0, int nb, const int* ells,
                                     const int* mms, int M, const double* qnm, int nq,
-                                    double dspin, int run_phenomd, int k0) {
+                                    double dspin, int run_phenomd) {
   const long long n = (long long)nb * M;
+  const int k0 = blockIdx.y * GRAD_CHUNK;
+  coeffs += blockIdx.y * n;
+  rmodes += blockIdx.y * n;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     const int bl = (int)(t / M), i = (int)(t % M);
@@ -127,8 +136,8 @@ __device__ inline PointTangents point_tangents(const ModeCoeffsT<GD>& c, const R
   return o;
 }
 
-// Sum of the GRAD_CHUNK partials over the block into out[k0 + k] for the directions < NGRAD.
-__device__ inline void block_reduce_grad(double* acc, double* out, int k0) {
+// Sum of the GRAD_CHUNK partials over the block into out[0 .. GRAD_CHUNK).
+__device__ inline void block_reduce_grad(double* acc, double* out) {
   __shared__ double red[GRAD_CHUNK][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
 #pragma unroll
@@ -138,35 +147,59 @@ __device__ inline void block_reduce_grad(double* acc, double* out, int k0) {
     if (lane == 0) red[k][w] = v;
   }
   __syncthreads();
-  if (threadIdx.x < GRAD_CHUNK && k0 + (int)threadIdx.x < NGRAD) {
+  if (threadIdx.x < GRAD_CHUNK) {
     double s = 0.0;
     for (int q = 0; q < nw; ++q) s += red[threadIdx.x][q];
-    out[k0 + threadIdx.x] = s;
+    out[threadIdx.x] = s;
   }
   __syncthreads();
 }
 
+// Modes per block of the contraction kernels: a binary's all where that gives blocks enough for
+// the GPU (each thread then takes several points: 2048 walkers, 128 bins: 4.5 ms, against 5.1 ms
+// with a block per mode), else one (128 binaries, 512 knots: 0.2 ms, against 0.4 ms).
+inline int contract_modes(int nb, int M) {
+  return (long long)nb * GRAD_PASSES >= 8ll * sm_count() ? M : 1;
+}
+inline int contract_blocks(int nb, int M, int mg) {
+  return std::min(nb * ((M + mg - 1) / mg), sm_count() * 16);
+}
+
+// grad[b0 + bl][k] = sum of part [GRAD_PASSES][nb][G][GRAD_CHUNK] over the G mode groups, in order.
+static __global__ void k_grad_sum(double* grad, const double* part, int b0, int nb, int G) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nb * NGRAD; t += gridDim.x * blockDim.x) {
+    const int bl = t / NGRAD, k = t - bl * NGRAD;
+    const double* p = part + ((size_t)(k / GRAD_CHUNK) * nb + bl) * G * GRAD_CHUNK + k % GRAD_CHUNK;
+    double v = 0.0;
+    for (int g = 0; g < G; ++g) v += p[(size_t)g * GRAD_CHUNK];
+    grad[(size_t)(b0 + bl) * NGRAD + k] = v;
+  }
+}
+
 // Heterodyne contraction: grad[b] = sum_{mode, j, channel} Re(gh[b, c, j] dW_c/dtheta) over
 // the sparse grid freqs[j] (lnL depends on h = sum_modes conj(W), and dL = Re(gh dW)).
-// One CTA per binary of [b0, b0 + nb); records indexed relative to b0.
-static __global__ void k_contract_het(double* grad, const ModeCoeffsT<GD>* coeffs,
+// One CTA per (binary of [b0, b0 + nb), group of mg modes) and pass, its sum into part
+// (k_grad_sum); records indexed relative to b0.
+static __global__ void k_contract_het(double* part, const ModeCoeffsT<GD>* coeffs,
                                       const ResponseModeT<GD>* rmodes, OrbitTables orb,
                                       const double* P, int B, int b0, int nb,
                                       const double* t_start, const double* t_end, double t_init,
                                       const double* freqs, const cplx* gh, int TDItag,
-                                      int rescaled, int tdi2, int M, int L, int k0) {
-  for (int bl = blockIdx.x; bl < nb; bl += gridDim.x) {
+                                      int rescaled, int tdi2, int M, int L, int mg) {
+  const int k0 = blockIdx.y * GRAD_CHUNK, ng = (M + mg - 1) / mg;
+  for (int r = blockIdx.x; r < nb * ng; r += gridDim.x) {
+    const int bl = r / ng, m0 = (r - bl * ng) * mg;
+    const size_t rec = ((size_t)blockIdx.y * nb + bl) * M + m0;
     const int b = b0 + bl;
     const GD t_ref = seed(P[11 * (size_t)B + b], 10, k0);
     const double ts = t_start[b], te = t_end[b];
     double acc[GRAD_CHUNK];
 #pragma unroll
     for (int k = 0; k < GRAD_CHUNK; ++k) acc[k] = 0.0;
-    for (int p = threadIdx.x; p < M * L; p += blockDim.x) {
-      const int m = p / L, j = p % L;
-      const PointTangents o =
-          point_tangents(coeffs[(size_t)bl * M + m], rmodes[(size_t)bl * M + m], orb, freqs[j],
-                         t_ref, t_init, TDItag, rescaled, tdi2);
+    for (int p = threadIdx.x; p < min(mg, M - m0) * L; p += blockDim.x) {
+      const int m = p / L, j = p - m * L;
+      const PointTangents o = point_tangents(coeffs[rec + m], rmodes[rec + m], orb, freqs[j], t_ref,
+                                             t_init, TDItag, rescaled, tdi2);
       if (!tf_gate(o.tf, ts, te)) continue;
 #pragma unroll
       for (int ch = 0; ch < 3; ++ch) {
@@ -176,7 +209,7 @@ static __global__ void k_contract_het(double* grad, const ModeCoeffsT<GD>* coeff
           acc[k] += u.re * o.W[ch].re.d[k] - u.im * o.W[ch].im.d[k];
       }
     }
-    block_reduce_grad(acc, grad + (size_t)b * NGRAD, k0);
+    block_reduce_grad(acc, part + ((size_t)blockIdx.y * nb * ng + r) * GRAD_CHUNK);
   }
 }
 
@@ -186,25 +219,28 @@ static __global__ void k_contract_het(double* grad, const ModeCoeffsT<GD>* coeff
 // the six transfer components; t(f), p = 2, only gates) and x_i the knots.  The knots move
 // with theta through the observation-window regrid: d x_i = x_i ((1 - r_i) wlo + r_i whi),
 // r_i = i / (L - 1), with (wlo, whi) = (d flo / flo, d fhi / fhi) of the row from
-// k_regrid_tangents (wreg [nb * M][2][GRAD_CHUNK], local rows); q_p is differentiated along the
-// moving knot (the frequency is a dual carrying d x_i).
-static __global__ void k_contract_direct(double* grad, const ModeCoeffsT<GD>* coeffs,
+// k_regrid_tangents (wreg [passes][nb * M][2][GRAD_CHUNK], local rows); q_p is differentiated along
+// the moving knot (the frequency is a dual carrying d x_i).  CTAs and part as k_contract_het.
+static __global__ void k_contract_direct(double* part, const ModeCoeffsT<GD>* coeffs,
                                          const ResponseModeT<GD>* rmodes, OrbitTables orb,
                                          const double* P, int B, int b0, int nb, double t_init,
                                          const double* x, const double* ybar, const double* xbar,
                                          const double* wreg, int TDItag, int rescaled, int tdi2,
-                                         int M, int L, int k0) {
+                                         int M, int L, int mg) {
+  const int k0 = blockIdx.y * GRAD_CHUNK, ng = (M + mg - 1) / mg;
   const size_t n = (size_t)B * M * L;
   const double inv_span = 1.0 / (double)(L - 1);
-  for (int bl = blockIdx.x; bl < nb; bl += gridDim.x) {
+  for (int rw = blockIdx.x; rw < nb * ng; rw += gridDim.x) {
+    const int bl = rw / ng, m0 = (rw - bl * ng) * mg;
+    const size_t rec = ((size_t)blockIdx.y * nb + bl) * M + m0;
     const int b = b0 + bl;
     const GD t_ref = seed(P[11 * (size_t)B + b], 10, k0);
     double acc[GRAD_CHUNK];
 #pragma unroll
     for (int k = 0; k < GRAD_CHUNK; ++k) acc[k] = 0.0;
-    for (int p = threadIdx.x; p < M * L; p += blockDim.x) {
-      const int m = p / L, i = p % L;
-      const size_t o = ((size_t)b * M + m) * L + i;
+    for (int p = threadIdx.x; p < min(mg, M - m0) * L; p += blockDim.x) {
+      const int m = p / L, i = p - m * L;
+      const size_t o = ((size_t)b * M + m0 + m) * L + i;
       const double w0 = ybar[o], w1 = ybar[n + o], xb = xbar[o];
       double wt[6];
       bool any = (w0 != 0.0) || (w1 != 0.0) || (xb != 0.0);
@@ -214,14 +250,14 @@ static __global__ void k_contract_direct(double* grad, const ModeCoeffsT<GD>* co
         any = any || (wt[q] != 0.0);
       }
       if (!any) continue;
-      const double* wr = wreg + ((size_t)bl * M + m) * 2 * GRAD_CHUNK;
+      const double* wr = wreg + (rec + m) * 2 * GRAD_CHUNK;
       const double r = i * inv_span;
       GD fk(x[o]);
 #pragma unroll
       for (int k = 0; k < GRAD_CHUNK; ++k)
         fk.d[k] = x[o] * ((1.0 - r) * wr[k] + r * wr[GRAD_CHUNK + k]);
-      const PointTangents pt = point_tangents(coeffs[(size_t)bl * M + m], rmodes[(size_t)bl * M + m],
-                                              orb, fk, t_ref, t_init, TDItag, rescaled, tdi2);
+      const PointTangents pt = point_tangents(coeffs[rec + m], rmodes[rec + m], orb, fk, t_ref,
+                                              t_init, TDItag, rescaled, tdi2);
 #pragma unroll
       for (int k = 0; k < GRAD_CHUNK; ++k) {
         double v = w0 * pt.amp.d[k] + w1 * pt.phase.d[k] + xb * fk.d[k];
@@ -231,7 +267,7 @@ static __global__ void k_contract_direct(double* grad, const ModeCoeffsT<GD>* co
         acc[k] += v;
       }
     }
-    block_reduce_grad(acc, grad + (size_t)b * NGRAD, k0);
+    block_reduce_grad(acc, part + ((size_t)blockIdx.y * nb * ng + rw) * GRAD_CHUNK);
   }
 }
 

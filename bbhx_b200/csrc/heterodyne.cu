@@ -140,7 +140,7 @@ using namespace bbhx;
 
 namespace {
 constexpr int kHetMaxL = 2048;
-constexpr int kGradChunk = 4096;  // walkers per dual-number setup / contraction batch
+constexpr int kGradChunk = 1024;  // walkers per dual-number setup / contraction batch (all passes)
 }
 
 namespace bbhx {
@@ -232,11 +232,13 @@ int bbhx_hdyn_grad(void* orbits, void* d_h, void* h_h, double* grad, const void*
   cplx* gh = nullptr;
   ModeCoeffsT<GD>* cD = nullptr;
   ResponseModeT<GD>* rD = nullptr;
+  double* gpart = nullptr;
   const int chunk = std::min(num_bin_all, kGradChunk);
-  const int nsm = sm_count();
+  const size_t nrec = (size_t)chunk * num_modes * GRAD_PASSES;
   if (pool_alloc((void**)&gh, sizeof(cplx) * 3 * (size_t)length * num_bin_all, s) != cudaSuccess ||
-      pool_alloc((void**)&cD, sizeof(ModeCoeffsT<GD>) * (size_t)chunk * num_modes, s) != cudaSuccess ||
-      pool_alloc((void**)&rD, sizeof(ResponseModeT<GD>) * (size_t)chunk * num_modes, s) != cudaSuccess) {
+      pool_alloc((void**)&cD, sizeof(ModeCoeffsT<GD>) * nrec, s) != cudaSuccess ||
+      pool_alloc((void**)&rD, sizeof(ResponseModeT<GD>) * nrec, s) != cudaSuccess ||
+      pool_alloc((void**)&gpart, sizeof(double) * nrec * GRAD_CHUNK, s) != cudaSuccess) {
     set_error("device allocation of the gradient scratch failed");
     st = ERR_CUDA;
   }
@@ -250,20 +252,25 @@ int bbhx_hdyn_grad(void* orbits, void* d_h, void* h_h, double* grad, const void*
     st = launch_het<false, true>(A, s);
     for (int b0 = 0; !st && b0 < num_bin_all; b0 += chunk) {
       const int nb = std::min(chunk, num_bin_all - b0);
-      const long long n = (long long)nb * num_modes;
-      for (int k0 = 0; !st && k0 < NGRAD; k0 += GRAD_CHUNK) {
-        k_grad_setup<<<grid_for(n, 64), 64, 0, s>>>(cD, rD, params, num_bin_all, b0, nb, ells,
-                                                    mms, num_modes, qnm_table, qnm_n, dspin,
-                                                    run_phenomd, k0);
-        st = launch_status("k_grad_setup");
-        if (st) break;
-        k_contract_het<<<(unsigned)std::min(nb, nsm * 8), 128, 0, s>>>(
-            grad, cD, rD, A.orb, params, num_bin_all, b0, nb, t_start, t_end, t_init, freqs, gh,
-            TDItag, rescaled, tdi2, num_modes, length, k0);
+      const int rows = nb * num_modes, mg = contract_modes(nb, num_modes);
+      k_grad_setup<<<dim3(grid_for(rows, 64), GRAD_PASSES), 64, 0, s>>>(
+          cD, rD, params, num_bin_all, b0, nb, ells, mms, num_modes, qnm_table, qnm_n, dspin,
+          run_phenomd);
+      st = launch_status("k_grad_setup");
+      if (!st) {
+        k_contract_het<<<dim3(contract_blocks(nb, num_modes, mg), GRAD_PASSES), 128, 0, s>>>(
+            gpart, cD, rD, A.orb, params, num_bin_all, b0, nb, t_start, t_end, t_init, freqs, gh,
+            TDItag, rescaled, tdi2, num_modes, length, mg);
         st = launch_status("k_contract_het");
+      }
+      if (!st) {
+        k_grad_sum<<<grid_for((long long)nb * NGRAD, 128), 128, 0, s>>>(
+            grad, gpart, b0, nb, (num_modes + mg - 1) / mg);
+        st = launch_status("k_grad_sum");
       }
     }
   }
+  if (gpart) pool_free(gpart, s);
   if (rD) pool_free(rD, s);
   if (cD) pool_free(cD, s);
   if (gh) pool_free(gh, s);

@@ -213,7 +213,7 @@ constexpr int FD_WARP_BINS = 32 * FD_K;          // 128
 // 512 -> 104 ms, 1024 -> 88, 2048 -> 80, 4096 -> 78, 8192 -> 79 ms mixed)
 constexpr int FD_TILE = 4096;
 // spline segments per (tile, mode) staged in shared memory: 8 for the mixed form, 4 for the
-// FP64 form, whose slices (FP64 coefficients plus the phase-recurrence state) must stay small
+// FP64 form, whose slices must stay small
 // enough for 3 CTAs per SM
 template <typename R>
 constexpr int fd_nseg() { return sizeof(R) == 8 ? 4 : 8; }
@@ -249,7 +249,7 @@ struct FusedArgs {
   // written at gh[3 (gh_off[b] + i - sup_start[b]) + channel]; null in the likelihood calls
   cplx* gh;
   const long long* gh_off;
-  // uniform-grid record of data_freqs (k_grid_detect), or null: panels / phase recurrence
+  // uniform-grid record of data_freqs (k_grid_detect), or null
   const struct GridInfo* grid;
   // work-queue counter, zero at launch: warps claim (tile, binary) items from it in increasing
   // order (claim_item)
@@ -260,7 +260,7 @@ struct FusedArgs {
 // BBHx's data streams take.  k_grid_detect verifies the form bit-exactly on the device for
 // three candidates of df (the rounded f[N-1] / (k0 + N - 1) and its two neighbours); bit c of
 // ok says candidate c reproduces every f_i.  The kernels then know every bin's exact frequency
-// k df (as p + pe, an error-free product), which panels and phase recurrence need.
+// k df (as p + pe, an error-free product), which the panels need.
 struct GridInfo {
   double k0;
   double df[3];
@@ -486,18 +486,11 @@ struct alignas(16) WarpStage {
 // (stride h = 32 df on a uniform grid) e^{i phi} advances by complex rotations:
 //   E_{j+1} = E_j R_j,  R_{j+1} = R_j Q_j,  Q_{j+1} = Q_j P,
 // with R = e^{i Delta}, Q = e^{i Delta^2}, P = e^{i Delta^3} the first, second and (constant)
-// third differences of the phase cubic.  Three FP64 complex products per bin replace the
-// per-bin phase cubic, range reduction and polynomial sine / cosine.  The state is re-anchored
-// (rot_anchor) at a mode's first chunk of a work item and wherever the chunk's segment changes;
-// an item holds at most kRecChunks chunks, so no lane runs more than kRecChunks * FD_K steps
-// from its anchor.  The anchor phase is
-// evaluated at the bin's exact frequency k df (error-free product) with a compensated final sum,
-// so it carries < 1e-13 rad instead of the ~ulp(phi) ~ 1e-10 - 1e-9 rad of a plain FP64
-// evaluation, and the products add ~2e-11 rad over the kRecChunks * FD_K = 128 steps between
-// anchors (bounded by the self-test against 50-digit phases: k_selftest_recurrence).
-constexpr int kRecChunks = 32;  // chunks (of FD_K steps per lane) between anchors, at most
-static_assert(FD_MAXCHUNK <= kRecChunks, "a work item must not run the recurrence longer");
-
+// third differences of the phase cubic.  The anchor phase is evaluated at the bin's exact
+// frequency k df (error-free product) with a compensated final sum, so it carries < 1e-13 rad
+// instead of the ~ulp(phi) ~ 1e-10 - 1e-9 rad of a plain FP64 evaluation, and the products add
+// ~2e-11 rad over 128 steps.  No likelihood kernel runs it (the panels of direct_panel.cuh took
+// its place, with the same anchor arithmetic at their nodes); bbhx_selftest_recurrence does.
 struct Rot {
   double er, ei, rr, ri, qr, qi, pr, pi;
 };
@@ -533,87 +526,6 @@ __device__ __forceinline__ void rot_anchor(Rot& z, const double* pc, double xk, 
   sincos_cw(D3, &z.pi, &z.pr);
 }
 
-// The FD_K bins of one lane inside staged segment ka of mode m, with the phase from the
-// recurrence z (advanced past the last bin on return): conj(T A e^{i phi}) into acc; bins with
-// f < 0 (outside the support) or failing the t(f) gate (CHECK) contribute zero.  The cubics
-// are evaluated one quantity at a time for all FD_K bins, reading that quantity's four
-// coefficients from shared memory, which keeps few coefficients and partial values live.
-template <typename R, bool CHECK>
-__device__ __forceinline__ void accumulate_chunk_rec(const WarpStage<R>& S, int m, int ka,
-                                                     const double* f, double ts, double te,
-                                                     R (*acc)[6], Rot& z) {
-  const double xk = S.x[m][ka];
-  double u[FD_K];
-  bool g[FD_K];
-#pragma unroll
-  for (int j = 0; j < FD_K; ++j) {
-    u[j] = f[j] - xk;
-    g[j] = f[j] >= 0.0;
-  }
-  if (CHECK) {
-    const double2 lo = *reinterpret_cast<const double2*>(&S.pc[m][ka][1][0]);
-    const double2 hi = *reinterpret_cast<const double2*>(&S.pc[m][ka][1][2]);
-#pragma unroll
-    for (int j = 0; j < FD_K; ++j) {
-      const double tf = fma(fma(fma(hi.y, u[j], hi.x), u[j], lo.y), u[j], lo.x);
-      g[j] = g[j] && tf_gate(tf, ts, te);
-    }
-  }
-  // e^{i phi} of the FD_K bins from the recurrence
-  double er[FD_K], ei[FD_K];
-#pragma unroll
-  for (int j = 0; j < FD_K; ++j) {
-    er[j] = z.er;
-    ei[j] = z.ei;
-    cmul_inplace(z.er, z.ei, z.rr, z.ri);
-    cmul_inplace(z.rr, z.ri, z.qr, z.qi);
-    cmul_inplace(z.qr, z.qi, z.pr, z.pi);
-  }
-  auto cubic4 = [&](int a, R* v) {
-    R c[4];
-    if (sizeof(R) == 4) {
-      const float4 q = *reinterpret_cast<const float4*>(&S.ac[m][ka][a][0]);
-      c[0] = (R)q.x; c[1] = (R)q.y; c[2] = (R)q.z; c[3] = (R)q.w;
-    } else {
-      const double2 lo = *reinterpret_cast<const double2*>(&S.ac[m][ka][a][0]);
-      const double2 hi = *reinterpret_cast<const double2*>(&S.ac[m][ka][a][2]);
-      c[0] = (R)lo.x; c[1] = (R)lo.y; c[2] = (R)hi.x; c[3] = (R)hi.y;
-    }
-#pragma unroll
-    for (int j = 0; j < FD_K; ++j) {
-      const R ur = (R)u[j];
-      v[j] = fma(fma(fma(c[3], ur, c[2]), ur, c[1]), ur, c[0]);
-    }
-  };
-  // A e^{i phi}
-  R apr[FD_K], api[FD_K];
-  {
-    R amp[FD_K];
-    cubic4(0, amp);
-#pragma unroll
-    for (int j = 0; j < FD_K; ++j) {
-      const R a = g[j] ? amp[j] : R(0);
-      apr[j] = a * (R)er[j];
-      api[j] = a * (R)ei[j];
-    }
-  }
-  // acc += conj(T_ch A e^{i phi}) channel by channel
-#pragma unroll
-  for (int ch = 0; ch < 3; ++ch) {
-    R tr[FD_K], ti[FD_K];
-    cubic4(1 + 2 * ch, tr);
-    cubic4(2 + 2 * ch, ti);
-#pragma unroll
-    for (int j = 0; j < FD_K; ++j) {
-      R* a = acc[j];
-      a[2 * ch] = fma(tr[j], apr[j], a[2 * ch]);
-      a[2 * ch] = fma(-ti[j], api[j], a[2 * ch]);
-      a[2 * ch + 1] = fma(-tr[j], api[j], a[2 * ch + 1]);
-      a[2 * ch + 1] = fma(-ti[j], apr[j], a[2 * ch + 1]);
-    }
-  }
-}
-
 // Self-test of the phase recurrence (no reference counterpart): thread l anchors at grid bin
 // k0 + l of the phase cubic pc = (y, c1, c2, c3) about knot xk (rot_anchor, step h = 32 df) and
 // advances `steps` times as the fused kernel does; out[2 (l steps + j) + {0, 1}] =
@@ -633,10 +545,10 @@ __global__ void k_selftest_recurrence(const double* pc, double xk, double k0, do
   }
 }
 
-// FP64 form off the recurrence path: one (bin, mode) with each quantity's cubic coefficients
+// FP64 form: one (bin, mode) with each quantity's cubic coefficients
 // read where they are used, from a staged segment in shared memory (SmemCoef) or from the
 // spline arrays in global memory (GlobalCoef), so these less frequent paths hold no segment in
-// registers and stay within the register budget of the recurrence path.
+// registers.
 struct SmemCoef {
   const WarpStage<double>& S;
   int m, k;
@@ -684,15 +596,6 @@ __device__ __forceinline__ void accumulate_bin_src(const Src& src, double f, dou
     acc[2 * ch + 1] -= tr * api + ti * apr;
   }
 }
-
-// Per-warp recurrence state: E, R, Q of every (mode, lane), P per mode and, per mode, the chunk
-// and segment the saved state belongs to.
-struct alignas(16) RecStage {
-  double2 st[FD_MAXM][3][32];  // E, R, Q of every lane
-  double2 P[FD_MAXM];          // e^{i Delta^3}: the same for every lane of a segment
-  int next_chunk[FD_MAXM];
-  int seg[FD_MAXM];
-};
 
 // G bins of one lane that lie in the same spline segment: the same arithmetic as
 // accumulate_bin, written branch-free (invalid or gated-off bins are dropped by selects) so the
@@ -800,42 +703,6 @@ __device__ __forceinline__ void load_seg(SegCoef<R>& cf, const WarpStage<R>& S, 
   }
 }
 
-// One (chunk, mode) on the phase recurrence: staged segment kl (global segment kg of the mode's
-// grid) holds every support bin of the chunk.  The saved state is continued when this mode's
-// previous chunk of the item was the one before, in the same segment; otherwise it is
-// re-anchored at this lane's first bin.
-template <typename R>
-__device__ __forceinline__ void rec_chunk_mode(const WarpStage<R>& S, RecStage* RS, int m, int kl,
-                                               int kg, int gate, int ck, int c0, int lane,
-                                               const double* fbin, double ts, double te,
-                                               R (*acc)[6], double gk0, double gdf, double hstep) {
-  const bool cont = (RS->next_chunk[m] == ck) && (RS->seg[m] == kg);
-  Rot z;
-  if (cont) {
-    const double2 e = RS->st[m][0][lane], r = RS->st[m][1][lane];
-    const double2 qq = RS->st[m][2][lane], pp = RS->P[m];
-    z.er = e.x; z.ei = e.y; z.rr = r.x; z.ri = r.y;
-    z.qr = qq.x; z.qi = qq.y; z.pr = pp.x; z.pi = pp.y;
-  } else {
-    rot_anchor(z, &S.pc[m][kl][0][0], S.x[m][kl], gk0 + (double)(c0 + lane), gdf, hstep);
-  }
-  const double2 pnew = make_double2(z.pr, z.pi);
-  if (gate == 1)
-    accumulate_chunk_rec<R, false>(S, m, kl, fbin, ts, te, acc, z);
-  else
-    accumulate_chunk_rec<R, true>(S, m, kl, fbin, ts, te, acc, z);
-  RS->st[m][0][lane] = make_double2(z.er, z.ei);
-  RS->st[m][1][lane] = make_double2(z.rr, z.ri);
-  RS->st[m][2][lane] = make_double2(z.qr, z.qi);
-  __syncwarp();
-  if (lane == 0) {
-    RS->next_chunk[m] = ck + 1;
-    RS->seg[m] = kg;
-    RS->P[m] = pnew;  // every lane's P of the segment is bitwise the same
-  }
-  __syncwarp();
-}
-
 // Copy segments [k0, k0 + n) of (binary b, mode m) into the mode's shared-memory slot: knots
 // x[k0 .. k0 + n], the FP64 phase / t(f) cubics and the amplitude / transfer cubics in R.
 template <typename R>
@@ -878,17 +745,16 @@ namespace bbhx {
 // functions, sin/cos of the reduced phase and the mode sum (the template) in FP32; the per-bin
 // products with data and weights in FP64 when the FP32 copies of data and weights are given
 // (the path of Likelihood and UnevenBatch), in FP32 without them.
-// GH (FP64 form only): also write d lnL / d h of every support bin to A.gh (gradient chain), with
-// the phase recurrence (state in RS) in the one-segment chunk path on uniform grids (A.grid).
+// GH (FP64 form only): also write d lnL / d h of every support bin to A.gh (gradient chain).
 // PANEL (FP64 form): uniform grids go to panel_item, with its shared memory in PS.
 template <bool MIXED, typename R, bool GH = false, bool PANEL = false>
 __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, WarpStage<R>& S,
-                                           RecStage* RS, PanelStage* PS, int lane) {
+                                           PanelStage* PS, int lane) {
   const long long BML = A.qstride;
   const int L = A.L;
   bool uni = false;
   double gk0 = 0.0, gdf = 0.0;
-  if ((GH || PANEL) && A.grid != nullptr) {
+  if (PANEL && A.grid != nullptr) {
     const unsigned ok = A.grid->ok & 7u;
     if (ok) {
       uni = true;
@@ -896,7 +762,6 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
       gdf = A.grid->df[(ok & 1u) ? 0 : (ok & 2u) ? 1 : 2];
     }
   }
-  const double hstep = 32.0 * gdf;
   {
     const int tile = (int)(q / A.B);
     const int b = (int)(q - (long long)tile * A.B);
@@ -914,7 +779,8 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
       if (uni) {
         const int2 kk = (lane < A.M) ? A.segtab[q * A.M + lane] : make_int2(0, 0);
         double dr = 0.0, di = 0.0, hh = 0.0;
-        panel_item(A, *PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, gk0, gdf, dr, di, hh);
+        panel_item<false>(A, *PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, gk0, gdf, dr, di,
+                          hh);
         for (int o = 16; o > 0; o >>= 1) {
           dr += __shfl_xor_sync(0xffffffffu, dr, o);
           di += __shfl_xor_sync(0xffffffffu, di, o);
@@ -931,7 +797,6 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
       }
     }
     // ---- stage this tile's segments for every mode
-    if (GH && lane < FD_MAXM) RS->next_chunk[lane] = -1;
     if (lane < A.M) {
       const int2 kk = A.segtab[q * A.M + lane];
       const int klo = max(kk.x, 0), khi = min(kk.y, L - 2);
@@ -999,10 +864,7 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
 #pragma unroll
       for (int j = 0; j < FD_K; ++j) {
         const int i = c0 + 32 * j + lane;
-        // on a verified uniform grid f_i = fl(k df) is recomputed bit-exactly instead of loaded
-        fbin[j] = (i >= s0 && i < s1) ? (uni ? __dmul_rn(gk0 + (double)i, gdf)
-                                             : __ldg(A.data_freqs + i))
-                                      : -1.0;
+        fbin[j] = (i >= s0 && i < s1) ? __ldg(A.data_freqs + i) : -1.0;
 #pragma unroll
         for (int c = 0; c < 6; ++c) acc[j][c] = R(0);
       }
@@ -1017,11 +879,6 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
           if (ka >= 0) {
             const int gate = S.gate[m][ka];
             if (gate == 2) continue;
-            if (GH && uni) {
-              rec_chunk_mode(S, RS, m, ka, S.klo[m] + ka, gate, ck, c0, lane, fbin, ts, te, acc,
-                             gk0, gdf, hstep);
-              continue;
-            }
             if constexpr (!MIXED) {
               const SmemCoef src{S, m, ka};
 #pragma unroll
@@ -1098,8 +955,7 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
             // next 32 knots, and stage a window of NSEG segments from there when the chunk
             // leaves the staged window
             const int ia = max(c0, s0), iz = min(c0 + FD_WARP_BINS, s1) - 1;
-            const double fa = uni ? __dmul_rn(gk0 + (double)ia, gdf) : __ldg(A.data_freqs + ia);
-            const double fz = uni ? __dmul_rn(gk0 + (double)iz, gdf) : __ldg(A.data_freqs + iz);
+            const double fa = __ldg(A.data_freqs + ia), fz = __ldg(A.data_freqs + iz);
             const int kc = S.kcur[m];
             const int kq = kc + lane;
             const double xv = (kq < L) ? __ldg(xrow + kq) : INFINITY;
@@ -1144,15 +1000,10 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
               if (ka == kz) {  // one segment holds every bin of the chunk
                 const int gate = S.gate[m][kl0];
                 if (gate != 2) {
-                  if (GH && uni) {
-                    rec_chunk_mode(S, RS, m, kl0, klo, gate, ck, c0, lane, fbin, ts, te, acc, gk0,
-                                   gdf, hstep);
-                  } else {
-                    const SmemCoef src{S, m, kl0};
+                  const SmemCoef src{S, m, kl0};
 #pragma unroll
-                    for (int j = 0; j < FD_K; ++j)
-                      if (fbin[j] >= 0.0) accumulate_bin_src(src, fbin[j], ts, te, acc[j]);
-                  }
+                  for (int j = 0; j < FD_K; ++j)
+                    if (fbin[j] >= 0.0) accumulate_bin_src(src, fbin[j], ts, te, acc[j]);
                 }
               } else {
                 int kb[FD_K];
@@ -1267,13 +1118,13 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
   }
 }
 
-// Shared memory of the fused kernels: FD_WARPS WarpStage slices, then (FP64 form, phase
-// recurrence) FD_WARPS RecStage slices.
-template <bool MIXED, bool GH = false>
+// Shared memory of the fused kernels: a WarpStage per warp, in the FP64 form of the uneven kernel
+// the same memory as a PanelStage.
+template <bool MIXED>
 constexpr size_t fused_smem_bytes() {
   using R = typename std::conditional<MIXED, float, double>::type;
-  constexpr size_t stage = sizeof(WarpStage<R>) + (GH ? sizeof(RecStage) : 0);
-  return FD_WARPS * (MIXED || stage > sizeof(PanelStage) ? stage : sizeof(PanelStage));
+  return FD_WARPS * (MIXED || sizeof(WarpStage<R>) > sizeof(PanelStage) ? sizeof(WarpStage<R>)
+                                                                        : sizeof(PanelStage));
 }
 
 template <bool MIXED, bool GH = false>
@@ -1284,14 +1135,15 @@ __global__ void __launch_bounds__(FD_WARPS * 32, MIXED ? 4 : 3) k_direct_fused(F
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   WarpStage<R>& S = reinterpret_cast<WarpStage<R>*>(smem_raw)[warp];
-  RecStage* RS = reinterpret_cast<RecStage*>(smem_raw + FD_WARPS * sizeof(WarpStage<R>)) + warp;
-  if (!MIXED && !GH && (A.grid->ok & 7u)) return;  // k_direct_panel's
+  if (!MIXED && (A.grid->ok & 7u)) return;  // k_direct_panel's
   const long long nitems = (long long)A.ntiles * A.B;
   for (long long q = claim_item(A.next, lane); q < nitems; q = claim_item(A.next, lane))
-    fused_item<MIXED, R, GH>(A, q, S, RS, nullptr, lane);
+    fused_item<MIXED, R, GH>(A, q, S, nullptr, lane);
 }
 
 // FP64 form on uniform grids (panel_item); returns at once on others, which k_direct_fused takes.
+// GH: also d lnL / d h of every bin (gradient chain).
+template <bool GH>
 __global__ void __launch_bounds__(FD_WARPS * 32, 3) k_direct_panel(FusedArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const unsigned ok = A.grid->ok & 7u;
@@ -1311,7 +1163,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32, 3) k_direct_panel(FusedArgs A) 
     double dr = 0.0, di = 0.0, hh = 0.0;
     if (t0 < s1 && t0 + A.tile > s0) {
       const int2 kk = (lane < A.M) ? A.segtab[q * A.M + lane] : make_int2(0, 0);
-      panel_item(A, PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, k0, df, dr, di, hh);
+      panel_item<GH>(A, PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, k0, df, dr, di, hh);
       for (int o = 16; o > 0; o >>= 1) {
         dr += __shfl_xor_sync(0xffffffffu, dr, o);
         di += __shfl_xor_sync(0xffffffffu, di, o);
@@ -1388,8 +1240,7 @@ __global__ void k_het_response_setup_multi(const HetMulti* __restrict__ HM, long
 // An uneven batch in ONE persistent launch: the walkers of every heterodyned problem (one
 // warp item each, het_item) followed by the (tile, binary) items of every direct problem
 // (fused_item), enumerated as one range from which the warps claim items (claim_item).  Each warp owns a
-// shared-memory slot of `slot` bytes that holds either a direct item's staged segments (and
-// recurrence state) or a walker's records and residual strip; the problem's argument block is
+// shared-memory slot of `slot` bytes that holds either a direct item's staged segments or a walker's records and residual strip; the problem's argument block is
 // copied to shared memory when the warp moves to another problem.  HET = false compiles the
 // walker path out (batches without heterodyned problems): the mixed direct items then run
 // within 128 registers, 4 CTAs per SM; with walkers the mixed kernel takes the FP64 budget
@@ -1436,7 +1287,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32, (MIXED && !HET) ? 4 : 3)
         for (int i = lane; i < n8; i += 32) dst[i] = src[i];
         __syncwarp();
       }
-      fused_item<MIXED, R, false, !MIXED>(gcur[warp], qd - MA->off[g], S, nullptr, PS, lane);
+      fused_item<MIXED, R, false, !MIXED>(gcur[warp], qd - MA->off[g], S, PS, lane);
     }
   }
 }
@@ -1556,7 +1407,8 @@ int direct_fused_gh(cplx* gh, const long long* gh_off, double* d_h, double* h_h,
                     const double* t_start, const double* t_end, int M, int L, int B_all, int b0,
                     int nb, cudaStream_t s) {
   if (nb == 0) return OK;
-  const int ntiles = (N + FD_TILE - 1) / FD_TILE;
+  const int tile = fused_tile(N, nb, FD_TILE);
+  const int ntiles = (N + tile - 1) / tile;
   const long long nitems = (long long)ntiles * nb;
   const long long row0 = (long long)b0 * M * L;
   double* part = nullptr;
@@ -1568,7 +1420,7 @@ int direct_fused_gh(cplx* gh, const long long* gh_off, double* d_h, double* h_h,
                                      {(void**)&grid, sizeof(GridInfo)},
                                      {(void**)&next, sizeof(unsigned long long)}}));
   k_tile_segments<<<grid_for(nitems * M, 256, sm_count() * 64), 256, 0, s>>>(
-      segtab, x + row0, data_freqs, start + b0, len + b0, nb, M, L, ntiles, FD_TILE);
+      segtab, x + row0, data_freqs, start + b0, len + b0, nb, M, L, ntiles, tile);
   int st = launch_status("k_tile_segments");
   if (!st) st = detect_grid(data_freqs, N, grid, s);
   if (!st) {
@@ -1590,7 +1442,7 @@ int direct_fused_gh(cplx* gh, const long long* gh_off, double* d_h, double* h_h,
     A.M = M;
     A.L = L;
     A.ntiles = ntiles;
-    A.tile = FD_TILE;
+    A.tile = tile;
     A.partials = part;
     A.segtab = segtab;
     A.d_h = nullptr;
@@ -1602,20 +1454,23 @@ int direct_fused_gh(cplx* gh, const long long* gh_off, double* d_h, double* h_h,
     A.gh_off = gh_off;
     A.grid = grid;
     A.next = next;
-    const size_t sm = fused_smem_bytes<false, true>();
-    st = cuda_status(cudaFuncSetAttribute(k_direct_fused<false, true>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
-                     "cudaFuncSetAttribute(k_direct_fused)");
+    st = cuda_status(cudaMemsetAsync(next, 0, sizeof(unsigned long long), s), "work-queue counter");
+    auto launch = [&](auto kernel, size_t sm, const char* what) {
+      int r = cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)sm),
+                          what);
+      if (!r) kernel<<<resident_grid(kernel, sm, nitems), FD_WARPS * 32, sm, s>>>(A);
+      return r ? r : launch_status(what);
+    };
+    // one of the two does the work, by the grid record
     if (!st)
-      st = cuda_status(cudaMemsetAsync(next, 0, sizeof(unsigned long long), s), "work-queue counter");
-    if (!st) {
-      const unsigned grid = resident_grid(k_direct_fused<false, true>, sm, nitems);
-      k_direct_fused<false, true><<<grid, FD_WARPS * 32, sm, s>>>(A);
-      st = launch_status("k_direct_fused (d lnL / d h)");
-    }
+      st = launch(k_direct_panel<true>, FD_WARPS * sizeof(PanelStage), "k_direct_panel (d lnL / d h)");
+    if (!st)
+      st = launch(k_direct_fused<false, true>, fused_smem_bytes<false>(),
+                  "k_direct_fused (d lnL / d h)");
   }
   if (!st && d_h != nullptr && h_h != nullptr) {
-    k_fused_reduce<<<grid_for(32LL * nb, 128), 128, 0, s>>>(part, start + b0, len + b0, nb, FD_TILE,
+    k_fused_reduce<<<grid_for(32LL * nb, 128), 128, 0, s>>>(part, start + b0, len + b0, nb, tile,
                                                             d_h + 2LL * b0, h_h + 2LL * b0);
     st = launch_status("k_fused_reduce");
   }
@@ -2083,7 +1938,7 @@ int bbhx_direct_like_fused(double* d_h, double* h_h, const double* data_freqs, c
       st = launch(k_direct_fused<true>, fused_smem_bytes<true>(),
                   "cudaFuncSetAttribute(k_direct_fused<true>)");
     if (!st && precision == 0) {  // one of the two does the work, by the grid record
-      st = launch(k_direct_panel, FD_WARPS * sizeof(PanelStage), "cudaFuncSetAttribute(k_direct_panel)");
+      st = launch(k_direct_panel<false>, FD_WARPS * sizeof(PanelStage), "cudaFuncSetAttribute(k_direct_panel)");
       if (!st) st = launch_status("k_direct_panel");
       if (!st)
         st = launch(k_direct_fused<false>, fused_smem_bytes<false>(),

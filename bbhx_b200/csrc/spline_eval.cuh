@@ -11,6 +11,22 @@ __device__ __forceinline__ bool tf_gate(double tf, double t_start, double t_end)
   return (tf >= t_start) && ((tf <= t_end) || (t_end <= 0.0));
 }
 
+// t(f) gate over a whole segment from the control points of its cubic (their hull holds it): 1 all
+// inside the observation window, 2 all outside, 0 undecided (per-bin gate).
+__device__ __forceinline__ int hull_gate(const double* c, double h, double ts, double te) {
+  const double a = c[1] * h, q = c[2] * h * h;
+  const double p1 = c[0] + a * (1.0 / 3.0);
+  const double p2 = c[0] + (2.0 * a + q) * (1.0 / 3.0);
+  const double p3 = c[0] + a + q + c[3] * h * h * h;
+  const double lo = fmin(fmin(c[0], p1), fmin(p2, p3));
+  const double hi = fmax(fmax(c[0], p1), fmax(p2, p3));
+  const double eps = 1e-6;  // s: far above the rounding of t(f) (~1e8 s)
+  if (!(lo == lo) || !(hi == hi)) return 0;
+  if (lo >= ts + eps && (te <= 0.0 || hi <= te - eps)) return 1;
+  if (hi < ts - eps || (te > 0.0 && lo > te + eps)) return 2;
+  return 0;
+}
+
 // conj(T_c * A e^{i phi}) for the three channels (WaveformBuild.cu:48-60)
 __device__ __forceinline__ void combine_channels(double amp, double phase, cplx T1, cplx T2,
                                                  cplx T3, cplx& h1, cplx& h2, cplx& h3) {
