@@ -115,13 +115,15 @@ def check(status, name=""):
 
 
 def call(name, *args):
-    check(getattr(lib(), name)(*args), name)
+    status = getattr(_lib or lib(), name)(*args)
+    if status:
+        check(status, name)
 
 
 def stream():
     import torch
 
-    return _VP(torch.cuda.current_stream().cuda_stream)
+    return _VP(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def dptr(t, dtype=None):

@@ -78,6 +78,8 @@ class LISATDIResponse:
         else:
             self._orbits = orbits
         self._orbits.configure(linear_interp_setup=True)
+        # time span the tables cover, for the checks of t(f)
+        self.t_span = float(self._orbits.t_base.min()), float(self._orbits.t_base.max())
 
     def _sanity_check_modes(self, ells, mms):
         for ell, mm in zip(ells, mms):

@@ -18,7 +18,7 @@ import numpy as np
 
 from . import _lib
 from .response.fastfdresponse import LISATDIResponse
-from .utils.arrays import atleast_1d, device, to_dev, to_np, torch
+from .utils.arrays import atleast_1d, device, param_rows, to_dev, to_np, torch
 from .utils.constants import YRSID_SI
 from .utils.interpolate import CubicSplineInterpolant
 from .waveforms.phenomhm import PhenomHMAmpPhase, step_front
@@ -110,9 +110,10 @@ class BBHWaveformFD:
         [2]) is given, the window-search failure and the orbit-coverage violation are
         recorded there instead of raising, so the caller can defer the host sync."""
         t = torch()
-        (m1, m2, chi1z, chi2z, distance, phi_ref, f_ref, inc, lam, beta, psi, t_ref) = params
         if freqs is None and length is None:
             raise ValueError("Must input freqs or length.")
+        (m1, m2, chi1z, chi2z, distance, phi_ref, f_ref, inc, lam, beta, psi,
+         t_ref) = param_rows(params)
         ap = self.amp_phase_gen
         if direct:
             length = freqs.shape[-1] if freqs is not None else length
@@ -156,7 +157,7 @@ class BBHWaveformFD:
                   rg.TDItag_int, int(rg.rescaled), int(rg.tdi2), M, length, B, _lib.stream())
         if not direct:
             tfs = out_buffer[2 * B * M * length:3 * B * M * length]
-            tmin, tmax = float(rg.orbits.t_base.min()), float(rg.orbits.t_base.max())
+            tmin, tmax = rg.t_span
             if flags is not None:
                 _lib.call("bbhx_tf_range_check", _lib.dptr(tfs), tfs.numel(), tmin, tmax,
                           _lib._VP(flags.data_ptr() + 4), _lib.stream())
@@ -240,7 +241,8 @@ class BBHWaveformFD:
         Returns the arguments of ``bbhx_hdyn_fused`` (after ``orbits``, before ``precision``)
         by name; the tensors stay referenced by the returned dict."""
         t = torch()
-        (m1, m2, chi1z, chi2z, distance, phi_ref, f_ref, inc, lam, beta, psi, t_ref) = params
+        (m1, m2, chi1z, chi2z, distance, phi_ref, f_ref, inc, lam, beta, psi,
+         t_ref) = param_rows(params)
         ap = self.amp_phase_gen
         pars, ts_d, te_d, _ = step_front(m1, m2, chi1z, chi2z, lam, beta, 1,
                                          (t_obs_start, t_obs_end), flags=flags)
