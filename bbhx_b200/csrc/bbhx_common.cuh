@@ -105,12 +105,6 @@ template <typename T>
 __host__ __device__ __forceinline__ cplxT<T> times_i(const cplxT<T>& a) {
   return {-a.im, a.re};
 }
-template <typename T>
-__device__ __forceinline__ cplxT<T> expi(const T& x) {
-  T s, c;
-  sincos(x, &s, &c);
-  return {c, s};
-}
 __device__ __forceinline__ double cabs(cplx a) { return hypot(a.re, a.im); }
 
 // Phase reduction to [-pi, pi]: k = rint(x / 2pi), then x - k*2pi with 2pi split into a
@@ -171,6 +165,16 @@ __device__ __forceinline__ void sincos_cw(double x, double* s, double* c, double
   double cc = (q & 1) ? sy : cy;
   *s = (q & 2) ? -ss : ss;
   *c = ((q + 1) & 2) ? -cc : cc;
+}
+
+// Sine and cosine in the per-point models: sincos_cw for plain FP64 (half the instructions of
+// CUDA's sincos with its large-argument branch), overloaded for the other scalar types.
+__device__ __forceinline__ void model_sincos(double x, double* s, double* c) { sincos_cw(x, s, c); }
+template <typename T>
+__device__ __forceinline__ cplxT<T> expi(const T& x) {
+  T s, c;
+  model_sincos(x, &s, &c);
+  return {c, s};
 }
 
 // sin / cos in FP32 of an FP64 angle: the quadrant reduction by pi/2 stays in FP64 (the

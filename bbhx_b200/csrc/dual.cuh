@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "bbhx_common.cuh"
+
 namespace bbhx {
 namespace ad {
 
@@ -197,6 +199,13 @@ template <int N>
 __device__ __forceinline__ void sincos(const Dual<N>& x, Dual<N>* s, Dual<N>* c) {
   double sv, cv;
   ::sincos(x.v, &sv, &cv);
+  *s = lin1(sv, cv, x);
+  *c = lin1(cv, -sv, x);
+}
+template <int N>
+__device__ __forceinline__ void model_sincos(const Dual<N>& x, Dual<N>* s, Dual<N>* c) {
+  double sv, cv;
+  sincos_cw(x.v, &sv, &cv);
   *s = lin1(sv, cv, x);
   *c = lin1(cv, -sv, x);
 }

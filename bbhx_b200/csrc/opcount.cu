@@ -78,6 +78,7 @@ __device__ __forceinline__ void sincos(const Cnt& x, Cnt* s, Cnt* c) {
   *s = Cnt(sv);
   *c = Cnt(cv);
 }
+__device__ __forceinline__ void model_sincos(const Cnt& x, Cnt* s, Cnt* c) { sincos(x, s, c); }
 __device__ __forceinline__ Cnt fabs(const Cnt& x) { tick(11); return Cnt(::fabs(x.v)); }
 __device__ __forceinline__ Cnt hypot(const Cnt& a, const Cnt& b) { tick(11); return Cnt(::hypot(a.v, b.v)); }
 __device__ __forceinline__ double floor(const Cnt& x) { tick(11); return ::floor(x.v); }

@@ -278,12 +278,17 @@ __device__ __forceinline__ T amp_int_ansatz(const PhenomDT<T>& d, T f) {
   return d.hc0 + u * (d.hc1 + u * (d.hc2 + (f - d.hf2) * (d.hc3 + (f - d.hf3) * d.hc4)));
 }
 
-// Full PhenomD amplitude (without the distance/mass scale), PhenomHMWaveform.cu:1508-1537
+// Full PhenomD amplitude (without the distance/mass scale), PhenomHMWaveform.cu:1508-1537; third =
+// Mf^(1/3)
 template <typename T>
-__device__ __forceinline__ T phenomd_amp(const PhenomDT<T>& d, T Mf) {
-  PowersT<T> p = make_powers(Mf);
-  T pre = d.amp0 / (Mf * p.sixth);
-  if (Mf < AMP_FJOIN_INS) return pre * amp_ins_ansatz(d, Mf, p);
+__device__ __forceinline__ T phenomd_amp(const PhenomDT<T>& d, T Mf, T* third) {
+  *third = cbrt(Mf);
+  const T pre = d.amp0 / (Mf * sqrt(*third));
+  if (Mf < AMP_FJOIN_INS) {
+    const T t = *third, t2 = t * t;  // powers t^2 .. t^9 by Horner
+    return pre * (1.0 + t2 * (d.ains[0] + t * (d.ains[1] + t * (d.ains[2] + t * (d.ains[3] +
+                  t * (d.ains[4] + t * (d.ains[5] + t * (d.ains[6] + t * d.ains[7]))))))));
+  }
   if (Mf >= d.fpeak) return pre * amp_mrd_ansatz(d, Mf);
   return pre * amp_int_ansatz(d, Mf);
 }
@@ -779,7 +784,7 @@ __device__ __forceinline__ T pn_habs(const ModeCoeffsT<T>& c, T v) {
                                         c.pn_delta * c.pn_Xs * (3427.0 / 1344 - c.pn_eta * 965 / 336) +
                                         c.pn_delta * (-PI)));
       const T im = c.pn_k * v4 * c.pn_delta * (-0.5 - 2.0 * 0.69314718056);
-      return hypot(re, im);
+      return sqrt(re * re + im * im);
     }
     case 2: return fabs(c.pn_k * (v * c.pn_delta));
     case 3: return fabs(c.pn_k * (v2 * (1.0 - 3.0 * c.pn_eta)));
@@ -793,15 +798,26 @@ __device__ __forceinline__ T pn_habs(const ModeCoeffsT<T>& c, T v) {
 // [P(Mf) / P(2Mf/m)] * [P_lm(Mfa) / P_22(Mfa)] with P = v^-3.5 |H(v)|, v = (2 pi x / m)^(1/3).
 // The v^-3.5 factors cancel exactly (v(2Mf/m) / v(Mf) = (2/m)^(1/3), v_22(Mfa) / v_lm(Mfa)
 // = (m/2)^(1/3)), leaving |H(v(Mf))| |H(v(Mfa))| / |H(v(2Mf/m))|; zero where |H(v(Mf))| = 0
-// (the reference's equal-mass guard).
+// (the reference's equal-mass guard).  All |H| but (2,1)'s are one power of v, whose ratio at the
+// two frequencies is a power of m/2, and v(Mfa) = (2 pi / m)^(1/3) Mfa^(1/3) reuses the cube root
+// of the amplitude (third_a).
 template <typename T>
-__device__ __forceinline__ T hm_amp_factor(const ModeCoeffsT<T>& c, T Mf, T Mfa) {
-  if (c.pn_case == 0) return 1.0;
-  const T t1 = pn_habs(c, cbrt(c.pn_2pi_m * Mf));
-  if (t1 == 0.0) return 0.0;
-  const T t2 = pn_habs(c, cbrt(c.pn_4pi_m2 * Mf));
-  const T h1 = pn_habs(c, cbrt(c.pn_2pi_m * Mfa));
-  return (t1 / t2) * h1;
+__device__ __forceinline__ T hm_amp_factor(const ModeCoeffsT<T>& c, T Mf, T third_a) {
+  switch (c.pn_case) {
+    case 0: return 1.0;
+    case 1: {  // m = 1
+      const T t = (Mf > c.am_fi) ? cbrt(Mf) : third_a * 0.7937005259840998;  // Mfa = 2 Mf
+      const T t1 = pn_habs(c, 1.8452701486440284 * t);
+      if (t1 == 0.0) return 0.0;
+      const T t2 = pn_habs(c, 2.324894703019253 * t);
+      return (t1 / t2) * pn_habs(c, 1.8452701486440284 * third_a);
+    }
+    case 2: return 1.1447142425533319 * pn_habs(c, 1.2794388617850085 * third_a);  // m = 3, v
+    case 3: return pn_habs(c, 1.4645918875615231 * third_a);                        // m = 2, v^2
+    case 4: return 1.5874010519681994 * pn_habs(c, 1.1624473515096265 * third_a);  // m = 4, v^2
+    case 5: return 1.5 * pn_habs(c, 1.2794388617850085 * third_a);                  // m = 3, v^3
+    default: return 0.0;
+  }
 }
 
 // Mapped PhenomD frequency and phase constants of the HM phase map (get_phase,
@@ -862,10 +878,13 @@ __device__ inline PointOutT<T> phm_eval_point(const ModeCoeffsT<T>& c, T f) {
   PointOutT<T> o;
   const T Mf = f * c.M_sec;
   if (c.phenomd_only) {
-    o.amp = phenomd_amp(c.d, Mf) * c.amp_scale;
+    T third;
+    o.amp = phenomd_amp(c.d, Mf, &third) * c.amp_scale;
   } else {
     const T Mfa = hm_amp_map(c, Mf);
-    o.amp = phenomd_amp(c.d, Mfa) * hm_amp_factor(c, Mf, Mfa) * c.amp_scale;
+    T third;
+    const T amp = phenomd_amp(c.d, Mfa, &third);
+    o.amp = amp * hm_amp_factor(c, Mf, third) * c.amp_scale;
   }
   mode_phase_tf(c, Mf, &o.phase, &o.tf);
   return o;

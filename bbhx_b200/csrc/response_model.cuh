@@ -163,20 +163,36 @@ struct TransferT {
 };
 using Transfer = TransferT<double>;
 
+// n H n of the symmetric mode matrix
 template <typename T>
 __device__ __forceinline__ cplxT<T> nHn(const cplxT<T>* H, const V3T<T>& n) {
-  T v[3] = {n.x, n.y, n.z};
-  cplxT<T> out = cmk(T(0.0), T(0.0));
-  for (int i = 0; i < 3; ++i) {
-    cplxT<T> t = cmk(T(0.0), T(0.0));
-    for (int j = 0; j < 3; ++j) t = t + H[i * 3 + j] * v[j];
-    out = out + v[i] * t;
-  }
-  return out;
+  const T xy = 2.0 * n.x * n.y, xz = 2.0 * n.x * n.z, yz = 2.0 * n.y * n.z;
+  const T xx = n.x * n.x, yy = n.y * n.y, zz = n.z * n.z;
+  return cmk(H[0].re * xx + H[4].re * yy + H[8].re * zz + H[1].re * xy + H[2].re * xz + H[5].re * yz,
+             H[0].im * xx + H[4].im * yy + H[8].im * zz + H[1].im * xy + H[2].im * xz + H[5].im * yz);
 }
 
 template <typename T>
 __device__ __forceinline__ T sinc(const T& x) { return x == 0.0 ? T(1.0) : sin(x) / x; }
+
+// x sinc(x (1 - kn)) and x sinc(x (1 + kn)) from (s1, c1) = sin, cos of x: the sines by the
+// addition theorem from one sine / cosine of x kn, the two divisions by one of 1 - kn^2 (a source
+// along the link, 1 - kn^2 -> 0, takes the plain form).
+template <typename T>
+__device__ __forceinline__ void sinc_pair(const T& x, const T& s1, const T& c1, const T& kn, T* minus,
+                                          T* plus) {
+  const T den = 1.0 - kn * kn;
+  if (!(den > 1e-6)) {
+    *minus = x * sinc(x * (1.0 - kn));
+    *plus = x * sinc(x * (1.0 + kn));
+    return;
+  }
+  T sk, ck;
+  model_sincos(x * kn, &sk, &ck);
+  const T inv = 1.0 / den, a = s1 * ck, b = c1 * sk;
+  *minus = (a - b) * ((1.0 + kn) * inv);
+  *plus = (a + b) * ((1.0 - kn) * inv);
+}
 
 // TDItag: 1 = XYZ, 2 = AET.  f in Hz, t in s.  The frequency has its own type F: double, or
 // the dual type T when the frequency itself carries tangents (knots that move with theta).
@@ -188,8 +204,8 @@ __device__ inline TransferT<T> response_point(const ResponseModeT<T>& r, const O
   // Roemer delay relative to the SSB (circular 1 AU orbit of the guiding centre)
   T al = Omega0 * t;
   T sa, ca;
-  sincos(al, &sa, &ca);
-  T kR = k[0] * (AU_SI * ca) + k[1] * (AU_SI * sa) + k[2] * (0.0 * t);
+  model_sincos(al, &sa, &ca);
+  T kR = AU_SI * (k[0] * ca + k[1] * sa);
   TransferT<T> out;
   out.phaseRdelay = 2. * PI / C_SI * f * kR;
 
@@ -204,28 +220,27 @@ __device__ inline TransferT<T> response_point(const ResponseModeT<T>& r, const O
   T kn2 = k[0] * n2.x + k[1] * n2.y + k[2] * n2.z;
   T kn3 = k[0] * n3.x + k[1] * n3.y + k[2] * n3.z;
   cplxT<T> n1H = nHn(r.H, n1), n2H = nHn(r.H, n2), n3H = nHn(r.H, n3);
-  T k12 = k[0] * (p1.x + p2.x) + k[1] * (p1.y + p2.y) + k[2] * (p1.z + p2.z);
-  T k23 = k[0] * (p2.x + p3.x) + k[1] * (p2.y + p3.y) + k[2] * (p2.z + p3.z);
-  T k31 = k[0] * (p3.x + p1.x) + k[1] * (p3.y + p1.y) + k[2] * (p3.z + p1.z);
   const double invL = orb.inv_armlength;
+  const T kp1 = k[0] * p1.x + k[1] * p1.y + k[2] * p1.z;
+  const T kp2 = k[0] * p2.x + k[1] * p2.y + k[2] * p2.z;
+  const T kp3 = k[0] * p3.x + k[1] * p3.y + k[2] * p3.z;
   T pre = f * orb.pi_L_over_c;
-  cplxT<T> e12 = expi(pre * (1. + k12 * invL));
-  cplxT<T> e23 = expi(pre * (1. + k23 * invL));
-  cplxT<T> e31 = expi(pre * (1. + k31 * invL));
-  // The constellation-centre phase factor exp(+i 2 pi f k.p0 / c) of the full response and
-  // the Roemer-delay factor exp(-i phaseRdelay) cancel identically (Response.cu:166,304-309).
-  cplxT<T> common = cmk(T(0.0), pre);
-  cplxT<T> c3 = common * n3H, c1 = common * n1H, c2 = common * n2H;
-  cplxT<T> G12 = c3 * (sinc(pre * (1. - kn3)) * e12);
-  cplxT<T> G21 = c3 * (sinc(pre * (1. + kn3)) * e12);
-  cplxT<T> G23 = c1 * (sinc(pre * (1. - kn1)) * e23);
-  cplxT<T> G32 = c1 * (sinc(pre * (1. + kn1)) * e23);
-  cplxT<T> G31 = c2 * (sinc(pre * (1. - kn2)) * e31);
-  cplxT<T> G13 = c2 * (sinc(pre * (1. + kn2)) * e31);
-
+  cplxT<T> e12 = expi(pre * (1. + (kp1 + kp2) * invL));
+  cplxT<T> e23 = expi(pre * (1. + (kp2 + kp3) * invL));
+  cplxT<T> e31 = expi(pre * (1. + (kp3 + kp1) * invL));
   // e^{ix}, x = pre, and its powers / sines from one sincos
   const cplxT<T> e1 = expi(pre);
   const cplxT<T> z = e1 * e1;  // e^{2ix}
+  // The constellation-centre phase factor exp(+i 2 pi f k.p0 / c) of the full response and
+  // the Roemer-delay factor exp(-i phaseRdelay) cancel identically (Response.cu:166,304-309).
+  const cplxT<T> c3 = times_i(n3H * e12), c1 = times_i(n1H * e23), c2 = times_i(n2H * e31);
+  T sm, sp;
+  sinc_pair(pre, e1.im, e1.re, kn3, &sm, &sp);
+  const cplxT<T> G12 = sm * c3, G21 = sp * c3;
+  sinc_pair(pre, e1.im, e1.re, kn1, &sm, &sp);
+  const cplxT<T> G23 = sm * c1, G32 = sp * c1;
+  sinc_pair(pre, e1.im, e1.re, kn2, &sm, &sp);
+  const cplxT<T> G31 = sm * c2, G13 = sp * c2;
   const T s2x = 2. * e1.im * e1.re;
   if (TDItag == 1) {
     cplxT<T> fac = rescaled ? cmk(T(1.0), T(0.0)) : times_i(2. * s2x * z);
