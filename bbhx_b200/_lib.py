@@ -45,6 +45,7 @@ _SIGS = {
     "bbhx_waveform_response_fused": [_VP] * 12 + [_D, _I, _I, _I, _I, _I, _I, _VP],
     "bbhx_interpolate": [_VP] * 6 + [_I] * 4 + [_VP],
     "bbhx_InterpTDI": [_VP] * 9 + [_I] * 4 + [_VP] * 3 + [_VP],
+    "bbhx_interp_templates": [_VP] * 9 + [_I] * 4 + [_VP] * 3,
     "bbhx_direct_sum": [_VP, _VP, _I, _I, _I, _I, _VP, _VP, _VP],
     "bbhx_fill_templates": [_VP, _VP, _VP, _VP, _I, _I, _I, _VP],
     "bbhx_direct_like": [_VP] * 7 + [_I, _I, _VP],

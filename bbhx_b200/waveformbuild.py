@@ -56,6 +56,10 @@ class TemplateInterpFD:
         self.num_channels = num_channels
         data_freqs = to_dev(data_freqs)
         (freqs, y, c1, c2, c3) = [to_dev(a) for a in interp_container]
+        ts = np.ascontiguousarray(to_np(t_start), dtype=np.float64)
+        te = np.ascontiguousarray(to_np(t_end), dtype=np.float64)
+        if num_channels == 3 and 1 <= num_modes <= 6 and length >= 2 and self.data_length:
+            return self._templates(data_freqs, freqs, y, c1, c2, c3, ts, te)
         freqs_shaped = freqs.reshape(num_bin_all, num_modes, -1)
         lo = freqs_shaped.reshape(num_bin_all, -1).min(dim=1).values
         hi = freqs_shaped.reshape(num_bin_all, -1).max(dim=1).values
@@ -72,13 +76,30 @@ class TemplateInterpFD:
         self.template_carrier = [t.zeros(int(num_channels * L), dtype=t.complex128, device=device())
                                  for L in lengths]
         tptrs = np.asarray([x.data_ptr() for x in self.template_carrier], dtype=np.int64)
-        ts = np.ascontiguousarray(to_np(t_start), dtype=np.float64)
-        te = np.ascontiguousarray(to_np(t_end), dtype=np.float64)
         self._inds = inds
         _lib.call("bbhx_InterpTDI", _lib.hptr(tptrs), _lib.dptr(data_freqs), _lib.dptr(freqs),
                   _lib.dptr(y), _lib.dptr(c1), _lib.dptr(c2), _lib.dptr(c3), _lib.hptr(ts),
                   _lib.hptr(te), length, self.data_length, num_bin_all, num_modes, _lib.hptr(ptrs),
                   _lib.hptr(start_inds), _lib.hptr(lengths), _lib.stream())
+        return self.template_channels
+
+    def _templates(self, data_freqs, freqs, y, c1, c2, c3, ts, te):
+        """The same templates by bbhx_interp_templates, which finds the bins' segments itself (the
+        index arrays and their searches took 40 % of an injection)."""
+        t = torch()
+        B, M, L = self.num_bin_all, self.num_modes, self.length
+        sup = t.empty(2 * B, dtype=t.int32, device=device())
+        _lib.call("bbhx_template_support", _lib.dptr(sup), _lib.dptr(sup[B:]), _lib.dptr(freqs), M,
+                  L, B, _lib.dptr(data_freqs), self.data_length, _lib.stream())
+        sup = to_np(sup)
+        self.start_inds, self.lengths = sup[:B].copy(), sup[B:].copy()
+        self.template_carrier = [t.empty(3 * int(n), dtype=t.complex128, device=device())
+                                 for n in self.lengths]
+        tptrs = np.asarray([x.data_ptr() for x in self.template_carrier], dtype=np.int64)
+        _lib.call("bbhx_interp_templates", _lib.hptr(tptrs), _lib.dptr(data_freqs),
+                  _lib.dptr(freqs), _lib.dptr(y), _lib.dptr(c1), _lib.dptr(c2), _lib.dptr(c3),
+                  _lib.hptr(ts), _lib.hptr(te), L, self.data_length, B, M,
+                  _lib.hptr(self.start_inds), _lib.hptr(self.lengths), _lib.stream())
         return self.template_channels
 
 

@@ -185,6 +185,16 @@ int bbhx_InterpTDI(const int64_t *template_ptrs, const double *data_freqs, const
                    int num_bin_all, int num_modes, const int64_t *inds_ptrs,
                    const int *inds_start, const int *ind_lengths, void *stream);
 
+/* Templates on the data grid from their splines, without index arrays (no reference counterpart
+ * as a call; the same result as InterpTDI over each binary's support): template_ptrs (device
+ * addresses of [3, lengths[b]] complex128), t_start, t_end, starts, lengths HOST arrays of
+ * num_bin_all entries; num_modes 1..6.  Synchronises the stream. */
+int bbhx_interp_templates(const int64_t *template_ptrs, const double *data_freqs, const double *x,
+                          const double *y, const double *c1, const double *c2, const double *c3,
+                          const double *t_start, const double *t_end, int length, int data_length,
+                          int num_bin_all, int num_modes, const int *starts, const int *lengths,
+                          void *stream);
+
 /* fill=True placement of per-binary templates on the data grid (replaces the Python slice
  * additions of src/bbhx/waveformbuild.py:663-693; no C counterpart there); template_ptrs,
  * starts, lengths are [host] arrays (device addresses of [3, len] complex128 templates);

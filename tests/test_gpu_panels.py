@@ -59,3 +59,60 @@ def test_panels_match_bin_by_bin(tobs, lo, hi, length, modes, batch, t_end):
     assert np.all(np.isfinite(dh)) and np.all(hh >= 0.0)
     assert np.all(np.abs(dh - dh1) <= eps * np.sqrt(uniform.d_d * hh1) + 1e-13)
     assert np.all(np.abs(hh - hh1) <= 2.0 * eps * hh1 + 1e-13)
+
+
+def _bin_by_bin(f, x, y, c, ts, te):
+    """Template [3, N] of one binary by plain torch: searchsorted segments, cubics, mode sum."""
+    import torch
+
+    M, L = x.shape
+    seg = torch.searchsorted(x, f[None].expand(M, -1).contiguous(), right=True) - 1
+    ok = (seg >= 0) & (seg < L - 1)
+    k = seg.clamp(0, L - 2)
+    u = f - torch.gather(x, 1, k)
+    v = [torch.gather(a, 2, k.expand(9, -1, -1)) for a in (y, *c)]
+    q = v[0] + u * (v[1] + u * (v[2] + u * v[3]))
+    ok = ok & (q[2] >= ts) & (q[2] <= te)
+    w = torch.where(ok, q[0], 0.0) * torch.exp(1j * q[1])
+    return torch.stack([torch.conj(torch.complex(q[3 + 2 * n], q[4 + 2 * n]) * w).sum(0)
+                        for n in range(3)])
+
+
+@pytest.mark.parametrize("tobs,lo,hi,length,modes,batch,nudge", [
+    (0.05, 1e-5, 0.1, 1024, None, 3, False),
+    (0.05, 1e-5, 0.1, 1024, None, 3, True),      # not k df: every bin searches its segment
+    (0.3, 5e-4, 0.03, 300, [(2, 2)], 1, False),
+    (0.1, 2e-2, 2.03e-2, 2000, [(3, 3), (4, 4)], 7, False),
+    (0.1, 2e-2, 2.0001e-2, 64, [(2, 1)], 2, True),
+])
+def test_templates_match_bin_by_bin(tobs, lo, hi, length, modes, batch, nudge):
+    """bbhx_interp_templates over whole supports against plain torch on the same splines.
+    Tolerance: both round phases of phi_max = 2 pi f t to FP64, ~8 ulp, on a template row's scale."""
+    import torch
+
+    from bbhx_b200 import BBHWaveformFD, EqualArmlengthOrbits
+    from bbhx_b200.synthetic import data_grid, draw_params
+
+    f = data_grid(tobs, lo, hi)
+    if nudge:
+        f[len(f) // 3] = np.nextafter(f[len(f) // 3], 1.0)
+    wave = BBHWaveformFD(response_kwargs=dict(orbits=EqualArmlengthOrbits(), TDItag="AET", tdi2=True))
+    P = draw_params(batch, tobs, 5 + length)
+    P[11] = np.random.default_rng(length).uniform(0.6, 0.9, batch) * tobs * YEAR
+    kw = dict(t_obs_start=0.0, t_obs_end=tobs, length=length, modes=modes)
+    got, starts, lens = wave(*P, freqs=f, **kw)
+    fd = torch.as_tensor(f, device="cuda")
+    buf, c1, c2, c3, x, ts, te = wave._spline_set(tuple(P), 0.0, tobs, length, modes)
+    B, M = batch, wave.num_modes
+    x, y, c1, c2, c3 = (a.reshape(-1, B, M, length) for a in (x, buf, c1, c2, c3))
+    eps = 8.0 * 2.0 ** -53 * 2.0 * np.pi * f[-1] * tobs * YEAR
+    for b in range(B):
+        st, n = int(starts[b]), int(lens[b])
+        a, z = (int(torch.searchsorted(fd, v.reshape(1), right=True)) for v in (x[0, b].min(), x[0, b].max()))
+        assert (st, n) == (a, z - a)
+        ref = _bin_by_bin(fd[st:st + n], x[0, b], y[:, b], (c1[:, b], c2[:, b], c3[:, b]), ts[b], te[b])
+        for c in range(3):
+            if n:
+                d = (got[b][c] - ref[c]).abs().max() / ref[c].abs().max()
+                print(b, c, float(d), eps)
+                assert d <= eps + 1e-12
