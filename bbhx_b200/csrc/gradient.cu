@@ -14,10 +14,9 @@
 //                     slopes' system K s = r is transposed and solved by the same cyclic
 //                     reduction (K^T lambda = s_bar), giving d lnL / d y at the knots
 //                     and d lnL / d x (the knots' positions, y held fixed)
-//   4. k_grad_setup + k_regrid_tangents + k_contract_direct: dual-number tangents of the
-//                     model at the knots and of the knots themselves (the observation-window
-//                     regrid moves them with theta), contracted with d lnL / d y and
-//                     d lnL / d x                                                  (forward)
+//   4. k_grad_setup + k_regrid_tangents + k_contract + k_grad_finish: derivatives of the model at
+//                     the knots and of the knots themselves (the observation-window regrid moves
+//                     them with theta), contracted with d lnL / d y and d lnL / d x
 #include <algorithm>
 #include <vector>
 
@@ -99,22 +98,6 @@ struct SplineRefs {
 // sums of those bins in registers; at the end of the segment one transposing reduction across
 // the warp (31 shuffles) leaves the total of moment l = (p, k) = (l / 4, l % 4) in lane l.
 constexpr int ADJ_THREADS = 128;
-
-// m[0..31] of every lane -> lane l returns the warp total of m[l] (recursive halving: at the
-// step of width w a lane keeps the half of its w values whose index bit matches its lane bit).
-__device__ __forceinline__ double warp_transpose_sum32(double (&m)[32], int lane) {
-#pragma unroll
-  for (int w = 16; w >= 1; w >>= 1) {
-    const bool upper = (lane & w) != 0;
-#pragma unroll
-    for (int i = 0; i < w; ++i) {
-      const double send = upper ? m[i] : m[i + w];
-      const double keep = upper ? m[i + w] : m[i];
-      m[i] = keep + __shfl_xor_sync(0xffffffffu, send, w);
-    }
-  }
-  return m[0];
-}
 
 __global__ void __launch_bounds__(ADJ_THREADS, 3)
 k_adj_coeffs(double* ybd, double* cb1, double* cb2, double* cb3, const cplx* gh,
@@ -386,16 +369,13 @@ __global__ void k_spline_adj(double* ybar, double* xbar, const double* ybd, cons
 // point's own frequency; To moves with lam and beta.  One thread per (local binary, mode)
 // repeats the forward's crossing search on the forward's default grid f0 and its t(f) tf0
 // ([B, M, L] each), evaluates the straddling points as duals and writes
-// wreg[pass][row][0][k] = d flo / flo and wreg[pass][row][1][k] = d fhi / fhi for the directions of
-// pass blockIdx.y.
-__global__ void k_regrid_tangents(double* wreg, const ModeCoeffsT<GD>* coeffs, const double* P,
+// wreg[row][0][k] = d log flo and wreg[row][1][k] = d log fhi (directions: kReg).
+using KD = ad::Dual<kIntr + 1>;  // the records of the contraction; the frequency's direction unused
+__global__ void k_regrid_tangents(double* wreg, const ModeCoeffsT<KD>* coeffs, const double* P,
                                   int B, int b0, int nb, int M, int L, const double* f0,
                                   const double* tf0, const double* t_start, const double* t_end,
                                   double tL_start, double tL_end) {
   const long long n = (long long)nb * M;
-  const int k0 = blockIdx.y * GRAD_CHUNK;
-  coeffs += blockIdx.y * n;
-  wreg += blockIdx.y * n * 2 * GRAD_CHUNK;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     const int bl = (int)(t / M), m = (int)(t % M);
@@ -403,36 +383,35 @@ __global__ void k_regrid_tangents(double* wreg, const ModeCoeffsT<GD>* coeffs, c
     const size_t row = ((size_t)b * M + m) * L;
     const double* f = f0 + row;
     const double* x = tf0 + row;
-    const ModeCoeffsT<GD>& c = coeffs[t];
-    const GD msum = seed(P[0 * (size_t)B + b], 0, k0) + seed(P[1 * (size_t)B + b], 1, k0);
-    const GD t_ref = seed(P[11 * (size_t)B + b], 10, k0);
+    const ModeCoeffsT<KD>& c = coeffs[t];
+    const double msum = P[b] + P[(size_t)B + b];
     // default-grid point j: f_j proportional to 1 / (m1 + m2)
     auto fdual = [&](int j) {
-      GD r(f[j]);
-#pragma unroll
-      for (int k = 0; k < GRAD_CHUNK; ++k) r.d[k] = -f[j] / msum.v * msum.d[k];
+      KD r(f[j]);
+      r.d[0] = r.d[1] = -f[j] / msum;
       return r;
     };
     // t(f_j) + t_ref along the moving point (value: the forward's)
     auto tdual = [&](int j) {
-      const GD fj = fdual(j);
-      GD ph, tf;
-      mode_phase_tf(c, fj * c.M_sec, &ph, &tf);
-      GD r = tf + t_ref;
-      r.v = x[j];
-      return r;
+      KD ph, tf;
+      mode_phase_tf(c, fdual(j) * c.M_sec, &ph, &tf);
+      tf.v = x[j];
+      return tf;
     };
-    // f where the chord of t(f) over [f_s, f_s+1] reaches T
-    auto cross = [&](int s, const GD& T) {
-      const GD fa = fdual(s), fb = fdual(s + 1), ta = tdual(s), tb = tdual(s + 1);
-      return (fb - fa) / (tb - ta) * (T - ta) + fa;
+    // f where the chord of t(f) over [f_s, f_s+1] reaches T; *dT = d f / d T = -d f / d t_ref
+    auto cross = [&](int s, double T, double* dT) {
+      const KD fa = fdual(s), fb = fdual(s + 1), ta = tdual(s), tb = tdual(s + 1);
+      const KD slope = (fb - fa) / (tb - ta);
+      *dT = slope.v;
+      return slope * (T - ta) + fa;
     };
     double tmin = x[0], tmax = x[0];
     for (int i = 1; i < L; ++i) {
       tmin = fmin(tmin, x[i]);
       tmax = fmax(tmax, x[i]);
     }
-    GD flo = fdual(0), fhi = fdual(L - 1);
+    KD flo = fdual(0), fhi = fdual(L - 1);
+    double lo_T = 0.0, hi_T = 0.0;
     if (tmin < 0.0) {
       int cnt = 0, seg = -1;
       for (int i = 0; i < L - 1; ++i)
@@ -440,26 +419,34 @@ __global__ void k_regrid_tangents(double* wreg, const ModeCoeffsT<GD>* coeffs, c
           if (cnt == 0) seg = i;
           ++cnt;
         }
-      if (cnt == 1) flo = cross(seg, GD(0.0));
+      if (cnt == 1) flo = cross(seg, 0.0, &lo_T);
     }
-    const GD lam = seed(P[8 * (size_t)B + b], 7, k0), beta = seed(P[9 * (size_t)B + b], 8, k0);
-    GD To = tssb_from_l(tL_end, lam, beta, 0.0) - tssb_from_l(tL_start, lam, beta, 0.0);
-    To.v = t_end[b] - t_start[b];  // the forward's span
-    if (tmax > To.v) {
+    const double To = t_end[b] - t_start[b];  // the forward's span
+    if (tmax > To) {
       int cnt = 0, seg = -1;
       for (int i = 0; i < L - 1; ++i)
-        if ((To.v < x[i + 1]) && (To.v > x[i])) {
+        if ((To < x[i + 1]) && (To > x[i])) {
           if (cnt == 0) seg = i;
           ++cnt;
         }
-      if (cnt == 1) fhi = cross(seg, To);
+      if (cnt == 1) fhi = cross(seg, To, &hi_T);
     }
-    double* w = wreg + (size_t)t * 2 * GRAD_CHUNK;
+    using AD = ad::Dual<2>;
+    const AD lam = seed<2>(P[8 * (size_t)B + b], 0), beta = seed<2>(P[9 * (size_t)B + b], 1);
+    const AD dTo = tssb_from_l(tL_end, lam, beta, 0.0) - tssb_from_l(tL_start, lam, beta, 0.0);
+    double* w = wreg + (size_t)t * 2 * kReg;
 #pragma unroll
-    for (int k = 0; k < GRAD_CHUNK; ++k) {
+    for (int k = 0; k < kIntr; ++k) {
       w[k] = flo.d[k] / flo.v;
-      w[GRAD_CHUNK + k] = fhi.d[k] / fhi.v;
+      w[kReg + k] = fhi.d[k] / fhi.v;
     }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      w[kIntr + k] = 0.0;
+      w[kReg + kIntr + k] = hi_T * dTo.d[k] / fhi.v;
+    }
+    w[kIntr + 2] = -lo_T / flo.v;
+    w[kReg + kIntr + 2] = -hi_T / fhi.v;
   }
 }
 
@@ -470,7 +457,6 @@ using namespace bbhx;
 namespace {
 constexpr long long kGhBudget = 1ll << 29;  // complex entries of d lnL / d h per batch (8 GB)
 constexpr int kDirectGradChunk = 512;  // binaries per batch of d lnL / d h
-constexpr int kDirectGradSub = 128;    // and per set of dual-number records (all passes at once)
 }  // namespace
 
 extern "C" {
@@ -520,17 +506,17 @@ int bbhx_direct_like_grad(void* orbits, void* d_h, void* h_h, double* grad, cons
   const bool moving = f_default != nullptr && tf_default != nullptr;
   double *ybd = nullptr, *cb = nullptr, *ybar = nullptr, *xbar = nullptr, *wreg = nullptr,
          *gpart = nullptr;
-  ModeCoeffsT<GD>* cD = nullptr;
-  ResponseModeT<GD>* rD = nullptr;
+  ModeCoeffsT<KD>* cD = nullptr;
+  ResponseModeT<RD>* rD = nullptr;
   const int chunk = std::min(B, kDirectGradChunk);
-  const int sub = std::min(B, kDirectGradSub);  // binaries per record set-up, all passes
-  const size_t nrec = (size_t)sub * M * GRAD_PASSES;
+  const int Q = contract_split(chunk, M, L);
+  const size_t nrec = (size_t)chunk * M;
   if (!st) {
-    const size_t nscratch = nall * 5 + (size_t)B * M * L + nrec * 3 * GRAD_CHUNK;
+    const size_t nscratch = nall * 5 + (size_t)B * M * L + nrec * (2 * kReg + 32 * (size_t)Q);
     // + one 8-byte word after the arrays: the work-queue counter of k_adj_coeffs
     if (pool_alloc((void**)&ybd, sizeof(double) * (nscratch + 1), s) != cudaSuccess ||
-        pool_alloc((void**)&cD, sizeof(ModeCoeffsT<GD>) * nrec, s) != cudaSuccess ||
-        pool_alloc((void**)&rD, sizeof(ResponseModeT<GD>) * nrec, s) != cudaSuccess) {
+        pool_alloc((void**)&cD, sizeof(*cD) * nrec, s) != cudaSuccess ||
+        pool_alloc((void**)&rD, sizeof(*rD) * nrec, s) != cudaSuccess) {
       set_error("device allocation of the gradient scratch failed");
       st = ERR_CUDA;
     }
@@ -540,10 +526,9 @@ int bbhx_direct_like_grad(void* orbits, void* d_h, void* h_h, double* grad, cons
     ybar = cb + 3 * nall;
     xbar = ybar + nall;
     wreg = xbar + (size_t)B * M * L;
-    gpart = wreg + nrec * 2 * GRAD_CHUNK;
-    // ybd / cb rows not written by k_adj_coeffs stay zero; wreg is zero for fixed knots
-    if (cudaMemsetAsync(ybd, 0, sizeof(double) * nall * 4, s) != cudaSuccess ||
-        cudaMemsetAsync(wreg, 0, sizeof(double) * nrec * 2 * GRAD_CHUNK, s) != cudaSuccess) {
+    gpart = wreg + nrec * 2 * kReg;
+    // ybd / cb rows not written by k_adj_coeffs stay zero
+    if (cudaMemsetAsync(ybd, 0, sizeof(double) * nall * 4, s) != cudaSuccess) {
       set_error("cudaMemsetAsync failed");
       st = ERR_CUDA;
     }
@@ -584,7 +569,7 @@ int bbhx_direct_like_grad(void* orbits, void* d_h, void* h_h, double* grad, cons
     if (!st) {
       const long long warps = (long long)nb * M * (L - 1);
       unsigned long long* next = reinterpret_cast<unsigned long long*>(
-          gpart + nrec * GRAD_CHUNK);
+          gpart + nrec * 32 * (size_t)Q);
       st = cuda_status(cudaMemsetAsync(next, 0, sizeof(unsigned long long), s),
                        "work-queue counter");
       // resident CTAs only: every warp claims segments until the queue drains (a segment holds
@@ -610,31 +595,28 @@ int bbhx_direct_like_grad(void* orbits, void* d_h, void* h_h, double* grad, cons
           ybar, xbar, ybd, cb, cb + nall, cb + 2 * nall, S, b0, nb);
       st = launch_status("k_spline_adj");
     }
-    for (int c0 = 0; !st && c0 < nb; c0 += sub) {
-      const int b1 = b0 + c0, n1 = std::min(sub, nb - c0);
-      const dim3 rows(grid_for((long long)n1 * M, 64), GRAD_PASSES);
-      k_grad_setup<<<rows, 64, 0, s>>>(cD, rD, params, B, b1, n1, ells, mms, M, qnm_table, qnm_n,
-                                       dspin, run_phenomd);
+    const unsigned rows = grid_for((long long)nb * M, 64);
+    if (!st) {
+      k_grad_setup<kIntr + 1><<<dim3(rows, 2), 64, 0, s>>>(cD, rD, params, B, b0, nb, ells, mms, M,
+                                                           qnm_table, qnm_n, dspin, run_phenomd);
       st = launch_status("k_grad_setup");
-      if (!st && moving) {
-        k_regrid_tangents<<<rows, 64, 0, s>>>(wreg, cD, params, B, b1, n1, M, L, f_default,
-                                              tf_default, t_start, t_end, t_obs_start_L,
-                                              t_obs_end_L);
-        st = launch_status("k_regrid_tangents");
-      }
-      if (!st) {
-        const int mg = contract_modes(n1, M);
-        k_contract_direct<<<dim3(contract_blocks(n1, M, mg), GRAD_PASSES), 128, 0, s>>>(
-            gpart, cD, rD, ((OrbitHandle*)orbits)->tab, params, B, b1, n1, t_init, x, ybar, xbar,
-            wreg, TDItag, rescaled, tdi2, M, L, mg);
-        st = launch_status("k_contract_direct");
-      }
-      if (!st) {
-        const int mg = contract_modes(n1, M);
-        k_grad_sum<<<grid_for((long long)n1 * NGRAD, 128), 128, 0, s>>>(grad, gpart, b1, n1,
-                                                                       (M + mg - 1) / mg);
-        st = launch_status("k_grad_sum");
-      }
+    }
+    if (!st && moving) {
+      k_regrid_tangents<<<rows, 64, 0, s>>>(wreg, cD, params, B, b0, nb, M, L, f_default,
+                                            tf_default, t_start, t_end, t_obs_start_L, t_obs_end_L);
+      st = launch_status("k_regrid_tangents");
+    }
+    if (!st) {
+      const ContractArgs<true> C{gpart, cD, rD, ((OrbitHandle*)orbits)->tab, params, B, b0, nb,
+                                 t_init, t_start, t_end, nullptr, nullptr, x, ybar, xbar,
+                                 TDItag, rescaled, tdi2, M, L, Q};
+      k_contract<true><<<contract_blocks(nb, M, Q), kContractWarps * 32, 0, s>>>(C);
+      st = launch_status("k_contract");
+    }
+    if (!st) {
+      k_grad_finish<<<grid_for((long long)nb * 32, 128), 128, 0, s>>>(
+          grad, gpart, rD, moving ? wreg : nullptr, params, B, b0, nb, M, Q);
+      st = launch_status("k_grad_finish");
     }
     if (gh) pool_free(gh, s);
     if (off) pool_free(off, s);

@@ -140,7 +140,7 @@ using namespace bbhx;
 
 namespace {
 constexpr int kHetMaxL = 2048;
-constexpr int kGradChunk = 1024;  // walkers per dual-number setup / contraction batch (all passes)
+constexpr int kGradChunk = 2048;  // walkers per record set-up and contraction (67 MB of records)
 }
 
 namespace bbhx {
@@ -216,8 +216,8 @@ int bbhx_hdyn_fused(void* orbits, void* d_h, void* h_h, const void* coeffs, cons
 
 // Heterodyned lnL and its gradient d lnL / d theta for the 11 parameters (order in
 // gradient_model.cuh) of B walkers: FP64 forward pass that also emits d lnL / d h at the
-// sparse grid (reverse part), then dual-number tangents of the waveform + response at every
-// (mode, frequency), contracted with those weights (forward part).  params: [12, B] device.
+// sparse grid, then the contraction of the model's tangents at every (mode, frequency) with those
+// weights (gradient_model.cuh).  params: [12, B] device.
 int bbhx_hdyn_grad(void* orbits, void* d_h, void* h_h, double* grad, const void* coeffs,
                    const double* params, const int* ells, const int* mms, const double* qnm_table,
                    int qnm_n, double dspin, double t_init, const double* t_start,
@@ -230,15 +230,16 @@ int bbhx_hdyn_grad(void* orbits, void* d_h, void* h_h, double* grad, const void*
   if (num_bin_all == 0) return OK;
   cudaStream_t s = (cudaStream_t)stream;
   cplx* gh = nullptr;
-  ModeCoeffsT<GD>* cD = nullptr;
-  ResponseModeT<GD>* rD = nullptr;
+  ModeCoeffsT<ad::Dual<kIntr>>* cD = nullptr;
+  ResponseModeT<RD>* rD = nullptr;
   double* gpart = nullptr;
   const int chunk = std::min(num_bin_all, kGradChunk);
-  const size_t nrec = (size_t)chunk * num_modes * GRAD_PASSES;
+  const int Q = contract_split(chunk, num_modes, length);
+  const size_t nrec = (size_t)chunk * num_modes;
   if (pool_alloc((void**)&gh, sizeof(cplx) * 3 * (size_t)length * num_bin_all, s) != cudaSuccess ||
-      pool_alloc((void**)&cD, sizeof(ModeCoeffsT<GD>) * nrec, s) != cudaSuccess ||
-      pool_alloc((void**)&rD, sizeof(ResponseModeT<GD>) * nrec, s) != cudaSuccess ||
-      pool_alloc((void**)&gpart, sizeof(double) * nrec * GRAD_CHUNK, s) != cudaSuccess) {
+      pool_alloc((void**)&cD, sizeof(*cD) * nrec, s) != cudaSuccess ||
+      pool_alloc((void**)&rD, sizeof(*rD) * nrec, s) != cudaSuccess ||
+      pool_alloc((void**)&gpart, sizeof(double) * nrec * Q * 32, s) != cudaSuccess) {
     set_error("device allocation of the gradient scratch failed");
     st = ERR_CUDA;
   }
@@ -252,21 +253,21 @@ int bbhx_hdyn_grad(void* orbits, void* d_h, void* h_h, double* grad, const void*
     st = launch_het<false, true>(A, s);
     for (int b0 = 0; !st && b0 < num_bin_all; b0 += chunk) {
       const int nb = std::min(chunk, num_bin_all - b0);
-      const int rows = nb * num_modes, mg = contract_modes(nb, num_modes);
-      k_grad_setup<<<dim3(grid_for(rows, 64), GRAD_PASSES), 64, 0, s>>>(
+      k_grad_setup<kIntr><<<dim3(grid_for((long long)nb * num_modes, 64), 2), 64, 0, s>>>(
           cD, rD, params, num_bin_all, b0, nb, ells, mms, num_modes, qnm_table, qnm_n, dspin,
           run_phenomd);
       st = launch_status("k_grad_setup");
       if (!st) {
-        k_contract_het<<<dim3(contract_blocks(nb, num_modes, mg), GRAD_PASSES), 128, 0, s>>>(
-            gpart, cD, rD, A.orb, params, num_bin_all, b0, nb, t_start, t_end, t_init, freqs, gh,
-            TDItag, rescaled, tdi2, num_modes, length, mg);
-        st = launch_status("k_contract_het");
+        const ContractArgs<false> C{gpart, cD, rD, A.orb, params, num_bin_all, b0, nb, t_init,
+                                    t_start, t_end, freqs, gh, nullptr, nullptr, nullptr,
+                                    TDItag, rescaled, tdi2, num_modes, length, Q};
+        k_contract<false><<<contract_blocks(nb, num_modes, Q), kContractWarps * 32, 0, s>>>(C);
+        st = launch_status("k_contract");
       }
       if (!st) {
-        k_grad_sum<<<grid_for((long long)nb * NGRAD, 128), 128, 0, s>>>(
-            grad, gpart, b0, nb, (num_modes + mg - 1) / mg);
-        st = launch_status("k_grad_sum");
+        k_grad_finish<<<grid_for((long long)nb * 32, 128), 128, 0, s>>>(
+            grad, gpart, rD, nullptr, params, num_bin_all, b0, nb, num_modes, Q);
+        st = launch_status("k_grad_finish");
       }
     }
   }

@@ -194,6 +194,32 @@ __device__ __forceinline__ void sinc_pair(const T& x, const T& s1, const T& c1, 
   *plus = (a + b) * ((1.0 - kn) * inv);
 }
 
+// Frequency factors of the three TDI channels (Response.cu:197-261), e1 = e^{ix}: X, Y, Z share
+// one; A, E, T carry their normalisations.
+template <typename T>
+__device__ __forceinline__ void tdi_factors(const cplxT<T>& e1, int TDItag, int rescaled, int tdi2,
+                                            cplxT<T> (&fac)[3]) {
+  const cplxT<T> one = cmk(T(1.0), T(0.0)), z = e1 * e1;
+  const T s2x = 2. * e1.im * e1.re;
+  if (TDItag == 1) {
+    fac[0] = fac[1] = fac[2] = rescaled ? one : times_i(2. * s2x * z);
+    return;
+  }
+  cplxT<T> fAE = one, fT = one;
+  if (!rescaled) {
+    fAE = times_i(SQRT2 * s2x * z);
+    fT = (2. * SQRT2 * s2x * e1.im) * (z * e1);
+  }
+  if (tdi2) {
+    const cplxT<T> f2 = times_i((-2. * (2. * s2x * z.re)) * (z * z));  // -2i sin4x e^{4ix}
+    fAE = f2 * fAE;
+    fT = f2 * fT;
+  }
+  fac[0] = fAE;
+  fac[1] = INVSQRT3 * fAE;
+  fac[2] = (2. * INVSQRT6) * fT;
+}
+
 // TDItag: 1 = XYZ, 2 = AET.  f in Hz, t in s.  The frequency has its own type F: double, or
 // the dual type T when the frequency itself carries tangents (knots that move with theta).
 template <typename T, typename F = double>
@@ -241,35 +267,19 @@ __device__ inline TransferT<T> response_point(const ResponseModeT<T>& r, const O
   const cplxT<T> G23 = sm * c1, G32 = sp * c1;
   sinc_pair(pre, e1.im, e1.re, kn2, &sm, &sp);
   const cplxT<T> G31 = sm * c2, G13 = sp * c2;
-  const T s2x = 2. * e1.im * e1.re;
+  cplxT<T> fac[3];
+  tdi_factors(e1, TDItag, rescaled, tdi2, fac);
   if (TDItag == 1) {
-    cplxT<T> fac = rescaled ? cmk(T(1.0), T(0.0)) : times_i(2. * s2x * z);
-    cplxT<T> X = G21 + z * G12 - G31 - z * G13;
-    cplxT<T> Y = G32 + z * G23 - G12 - z * G21;
-    cplxT<T> Z = G13 + z * G31 - G23 - z * G32;
-    out.L1 = fac * X;
-    out.L2 = fac * Y;
-    out.L3 = fac * Z;
+    out.L1 = fac[0] * (G21 + z * G12 - G31 - z * G13);
+    out.L2 = fac[1] * (G32 + z * G23 - G12 - z * G21);
+    out.L3 = fac[2] * (G13 + z * G31 - G23 - z * G32);
     return out;
   }
-  cplxT<T> fAE, fT;
-  if (rescaled) {
-    fAE = cmk(T(1.0), T(0.0));
-    fT = cmk(T(1.0), T(0.0));
-  } else {
-    fAE = times_i(SQRT2 * s2x * z);
-    fT = (2. * SQRT2 * s2x * e1.im) * (z * e1);
-  }
-  cplxT<T> one = cmk(T(1.0), T(0.0));
-  cplxT<T> A = 0.5 * ((one + z) * (G31 + G13) - G23 - z * G32 - G21 - z * G12);
-  cplxT<T> E = (0.5 * INVSQRT3) * ((one - z) * (G13 - G31) + (cmk(T(2.0), T(0.0)) + z) * (G12 - G32) +
-                              (one + 2. * z) * (G21 - G23));
-  cplxT<T> Tc = INVSQRT6 * (G21 - G12 + G32 - G23 + G13 - G31);
-  cplxT<T> f2 = cmk(T(2.0), T(0.0));
-  if (tdi2) f2 = 2.0 * times_i((-2. * (2. * s2x * z.re)) * (z * z));  // -2i sin4x e^{4ix}
-  out.L1 = f2 * (fAE * A);
-  out.L2 = f2 * (fAE * E);
-  out.L3 = f2 * (fT * Tc);
+  const cplxT<T> one = cmk(T(1.0), T(0.0));
+  out.L1 = fac[0] * ((one + z) * (G31 + G13) - G23 - z * G32 - G21 - z * G12);
+  out.L2 = fac[1] * ((one - z) * (G13 - G31) + (cmk(T(2.0), T(0.0)) + z) * (G12 - G32) +
+                     (one + 2. * z) * (G21 - G23));
+  out.L3 = fac[2] * (G21 - G12 + G32 - G23 + G13 - G31);
   return out;
 }
 
