@@ -215,17 +215,17 @@ __device__ __forceinline__ double spline_mbar(int j, const double* xs, int L, co
   const double tbar = -cb2[j] + cb3[j] / h;
   double v = (cb2[j] - 2.0 * tbar) / h;
   // interior rows r = 1..L-2: r_r = 3 (h_r m_{r-1} + h_{r-1} m_r)
-  if (j >= 1 && j <= L - 2) v += 3.0 * lam[j] * (xs[j] - xs[j - 1]);
-  if (j + 1 <= L - 2) v += 3.0 * lam[j + 1] * (xs[j + 2] - xs[j + 1]);
+  if (j >= 1 && j <= L - 2) v += 3.0 * lam[cr_slot(j)] * (xs[j] - xs[j - 1]);
+  if (j + 1 <= L - 2) v += 3.0 * lam[cr_slot(j + 1)] * (xs[j + 2] - xs[j + 1]);
   // row 0: r_0 = ((h0 + 2 d0) h1 m_0 + h0^2 m_1) / d0
   const double h0 = xs[1] - xs[0], h1 = xs[2] - xs[1], d0 = xs[2] - xs[0];
-  if (j == 0) v += lam[0] * (h0 + 2 * d0) * h1 / d0;
-  if (j == 1) v += lam[0] * h0 * h0 / d0;
+  if (j == 0) v += lam[cr_slot(0)] * (h0 + 2 * d0) * h1 / d0;
+  if (j == 1) v += lam[cr_slot(0)] * h0 * h0 / d0;
   // row L-1: r = (h_{L-2}^2 m_{L-3} + (2 dL + h_{L-2}) h_{L-3} m_{L-2}) / dL
   const double hl = xs[L - 1] - xs[L - 2], hp = xs[L - 2] - xs[L - 3];
   const double dL = xs[L - 1] - xs[L - 3];
-  if (j == L - 3) v += lam[L - 1] * hl * hl / dL;
-  if (j == L - 2) v += lam[L - 1] * (2 * dL + hl) * hp / dL;
+  if (j == L - 3) v += lam[cr_slot(L - 1)] * hl * hl / dL;
+  if (j == L - 2) v += lam[cr_slot(L - 1)] * (2 * dL + hl) * hp / dL;
   return v;
 }
 
@@ -235,16 +235,18 @@ __device__ __forceinline__ double spline_mbar(int j, const double* xs, int L, co
 // Forward: h_i = x_{i+1} - x_i, m_i = (y_{i+1} - y_i) / h_i; K(h) s = r(h, m); c1 = s_i,
 // t = (s_i + s_{i+1} - 2 m_i) / h_i, c2 = (m_i - s_i) / h_i - t, c3 = t / h_i; a data bin f of
 // segment i reads y_i + c1 u + c2 u^2 + c3 u^3 with u = f - x_i.  Shared memory: x, a, b, c,
-// d[9][L].
+// w, d[9] of cr_pad(L).
 __global__ void k_spline_adj(double* ybar, double* xbar, const double* ybd, const double* cb1,
                              const double* cb2, const double* cb3, SplineRefs S, int b0, int nb) {
   extern __shared__ double sm[];
   const int L = S.L;
   double* xs = sm;
-  double* a = xs + L;
-  double* bb = a + L;
-  double* c = bb + L;
-  double* d = c + L;
+  const int ld = cr_pad(L);
+  double* a = xs + ld;
+  double* bb = a + ld;
+  double* c = bb + ld;
+  double* w = c + ld;
+  double* d = w + ld;
   const int nsys = nb * S.M;
   for (int sys = blockIdx.x; sys < nsys; sys += gridDim.x) {
     const size_t row = (size_t)b0 * S.M + sys;
@@ -266,9 +268,10 @@ __global__ void k_spline_adj(double* ybar, double* xbar, const double* ybd, cons
       fwd(i, &ta, &tb, &tc);
       if (i > 0) fwd(i - 1, &pa, &pb, &pc); else pc = 0.0;
       if (i < L - 1) fwd(i + 1, &na, &nb_, &nc); else na = 0.0;
-      a[i] = (i > 0) ? pc : 0.0;
-      bb[i] = tb;
-      c[i] = (i < L - 1) ? na : 0.0;
+      const int j = cr_slot(i);
+      a[j] = (i > 0) ? pc : 0.0;
+      bb[j] = tb;
+      c[j] = (i < L - 1) ? na : 0.0;
       // right-hand sides: s_bar from the coefficient adjoints
       for (int p = 0; p < 9; ++p) {
         double sb = 0.0;
@@ -285,11 +288,11 @@ __global__ void k_spline_adj(double* ybar, double* xbar, const double* ybd, cons
             sb += tbar / h;
           }
         }
-        d[(size_t)p * L + i] = sb;
+        d[(size_t)p * ld + j] = sb;
       }
     }
     __syncthreads();
-    cr_solve(a, bb, c, d, L, 9, L);  // lambda = K^{-T} s_bar (r_bar)
+    cr_solve(a, bb, c, w, d, 9, L);  // lambda = K^{-T} s_bar (r_bar)
     // y_bar from m_bar
     for (int i = threadIdx.x; i < L; i += blockDim.x) {
       for (int p = 0; p < 9; ++p) {
@@ -298,7 +301,7 @@ __global__ void k_spline_adj(double* ybar, double* xbar, const double* ybd, cons
           ybar[o + i] = 0.0;
           continue;
         }
-        const double* lam = d + (size_t)p * L;
+        const double* lam = d + (size_t)p * ld;
         double yb = (i < L - 1) ? ybd[o + i] : 0.0;
         if (i < L - 1) yb -= spline_mbar(i, xs, L, lam, cb2 + o, cb3 + o) / (xs[i + 1] - xs[i]);
         if (i > 0) yb += spline_mbar(i - 1, xs, L, lam, cb2 + o, cb3 + o) / (xs[i] - xs[i - 1]);
@@ -315,7 +318,7 @@ __global__ void k_spline_adj(double* ybar, double* xbar, const double* ybd, cons
       for (int p = 0; p < 9; ++p) {
         if (p == 2) continue;
         const size_t o = (size_t)p * S.n + row * L;
-        const double* lam = d + (size_t)p * L;
+        const double* lam = d + (size_t)p * ld;
         const double* y = S.y + o;
         const double* s1 = S.c1 + o;
         auto hh = [&](int j) { return xs[j + 1] - xs[j]; };
@@ -330,20 +333,20 @@ __global__ void k_spline_adj(double* ybar, double* xbar, const double* ybd, cons
         e += s1[i] * ybd[o + i] + 2.0 * c2i * cb1[o + i] + 3.0 * c3i * cb2[o + i];
         hb -= (cb2[o + i] * c2i + 2.0 * cb3[o + i] * c3i) / h;
         hb -= spline_mbar(i, xs, L, lam, cb2 + o, cb3 + o) * mm(i) / h;
-        if (i >= 1 && i <= L - 2) hb += lam[i] * (3.0 * mm(i - 1) - sl(i - 1) - 2.0 * sl(i));
-        if (i <= L - 3) hb += lam[i + 1] * (3.0 * mm(i + 1) - 2.0 * sl(i + 1) - sl(i + 2));
+        if (i >= 1 && i <= L - 2) hb += lam[cr_slot(i)] * (3.0 * mm(i - 1) - sl(i - 1) - 2.0 * sl(i));
+        if (i <= L - 3) hb += lam[cr_slot(i + 1)] * (3.0 * mm(i + 1) - 2.0 * sl(i + 1) - sl(i + 2));
         if (i <= 1) {  // row 0: h1 s0 + d0 s1 = ((3 h0 + 2 h1) h1 m0 + h0^2 m1) / d0
           const double h0 = hh(0), h1 = hh(1), d0 = h0 + h1;
           const double rhs = ((3.0 * h0 + 2.0 * h1) * h1 * mm(0) + h0 * h0 * mm(1)) / d0;
-          if (i == 0) hb += lam[0] * ((3.0 * h1 * mm(0) + 2.0 * h0 * mm(1) - rhs) / d0 - sl(1));
-          else hb += lam[0] * (((3.0 * h0 + 4.0 * h1) * mm(0) - rhs) / d0 - sl(0) - sl(1));
+          if (i == 0) hb += lam[cr_slot(0)] * ((3.0 * h1 * mm(0) + 2.0 * h0 * mm(1) - rhs) / d0 - sl(1));
+          else hb += lam[cr_slot(0)] * (((3.0 * h0 + 4.0 * h1) * mm(0) - rhs) / d0 - sl(0) - sl(1));
         }
         if (i >= L - 3) {  // row L-1: dL s_{L-2} + A s_{L-1} = (Bh^2 m_{L-3} + (2A + 3Bh) A m_{L-2}) / dL
           const double A = hh(L - 3), Bh = hh(L - 2), dL = A + Bh;
           const double mq = mm(L - 3), mr = mm(L - 2);
           const double rhs = (Bh * Bh * mq + (2.0 * A + 3.0 * Bh) * A * mr) / dL;
-          if (i == L - 3) hb += lam[L - 1] * (((4.0 * A + 3.0 * Bh) * mr - rhs) / dL - sl(L - 2) - sl(L - 1));
-          else hb += lam[L - 1] * ((2.0 * Bh * mq + 3.0 * A * mr - rhs) / dL - sl(L - 2));
+          if (i == L - 3) hb += lam[cr_slot(L - 1)] * (((4.0 * A + 3.0 * Bh) * mr - rhs) / dL - sl(L - 2) - sl(L - 1));
+          else hb += lam[cr_slot(L - 1)] * ((2.0 * Bh * mq + 3.0 * A * mr - rhs) / dL - sl(L - 2));
         }
       }
       a[i] = e;
@@ -534,7 +537,7 @@ int bbhx_direct_like_grad(void* orbits, void* d_h, void* h_h, double* grad, cons
     }
   }
   const int nsm = sm_count();
-  const size_t smem = sizeof(double) * (size_t)(4 + 9) * L;
+  const size_t smem = sizeof(double) * (size_t)(5 + 9) * cr_pad(L);
   if (!st && cudaFuncSetAttribute(k_spline_adj, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)smem) != cudaSuccess) {
     set_error("cudaFuncSetAttribute failed for k_spline_adj");

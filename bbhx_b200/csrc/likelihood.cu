@@ -154,8 +154,26 @@ __global__ void k_hdyn(cplx* d_h, cplx* h_h, const cplx* __restrict__ r,
 // ---------------------------------------------------------------------------- fused direct
 // Support of each binary on the data grid (waveformbuild.py:136-177): [start, start+len) with
 // start = searchsorted(f, min x, 'right'), end = searchsorted(f, max x, 'right').
-// Support [start, start + len) on the data grid of binary b (whole block): the data bins in
-// [min x, max x] of its knots over all modes (searchsorted right of both ends).
+
+// Number of entries <= v of the sorted f[0..N) (searchsorted right) by a whole warp: 32 probes per
+// round, 5 rounds for 3 10^6 bins where one thread's bisection takes 22 dependent loads (supports of
+// one binary with 1024 knots per mode: 40 -> 28 us, most of it now the first pass over the knots).
+__device__ __forceinline__ int warp_count_le(const double* __restrict__ f, int N, double v) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0, hi = N;  // the answer lies in [lo, hi]
+  while (hi - lo > 32) {
+    const int step = (hi - lo + 31) / 32;
+    const long long i = (long long)lo + (long long)(lane + 1) * step - 1;
+    const int c = __popc(__ballot_sync(0xffffffffu, i < hi && f[i] <= v));
+    lo += c * step;
+    hi = min(hi, lo + step - 1);
+  }
+  const int i = lo + lane;
+  return lo + __popc(__ballot_sync(0xffffffffu, i < hi && f[i] <= v));
+}
+
+// Support [start, start + len) on the data grid of binary b (whole block, two warps or more): the
+// data bins in [min x, max x] of its knots over all modes.
 __device__ __forceinline__ void support_of(const double* __restrict__ x, int M, int L, int b,
                                            const double* __restrict__ data_freqs, int N,
                                            int* start, int* len) {
@@ -170,32 +188,26 @@ __device__ __forceinline__ void support_of(const double* __restrict__ x, int M, 
     hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   }
   __shared__ double slo[32], shi[32];
-  int w = threadIdx.x >> 5;
+  __shared__ int send;
+  const int w = threadIdx.x >> 5;
   if ((threadIdx.x & 31) == 0) {
     slo[w] = lo;
     shi[w] = hi;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
+  int n = 0;
+  if (w < 2) {  // warp 0 counts up to the lowest knot, warp 1 up to the highest
+    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) {
       lo = fmin(lo, slo[k]);
       hi = fmax(hi, shi[k]);
     }
-    // searchsorted right: number of entries <= v
-    int a = 0, c = N;
-    while (a < c) {
-      int mid = (a + c) >> 1;
-      if (data_freqs[mid] <= lo) a = mid + 1; else c = mid;
-    }
-    int s = a;
-    a = s;
-    c = N;
-    while (a < c) {
-      int mid = (a + c) >> 1;
-      if (data_freqs[mid] <= hi) a = mid + 1; else c = mid;
-    }
-    start[b] = s;
-    len[b] = a - s;
+    n = warp_count_le(data_freqs, N, w == 0 ? lo : hi);
+    if (threadIdx.x == 32) send = n;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    start[b] = n;
+    len[b] = max(send - n, 0);
   }
   __syncthreads();
 }
@@ -1372,36 +1384,42 @@ __global__ void k_fused_reduce_multi(const MultiArgs* __restrict__ MA) {
   }
 }
 
-// out: d_h[b], h_h[b] complex (device).  One warp per binary: lane l sums tiles l, l+32, ...
-// of the binary's support, then a fixed shuffle tree; the order is the same on every run.
+// out: d_h[b], h_h[b] complex (device).  One block per binary: thread l sums tiles l, l + 256, ...
+// of the binary's support, then fixed trees over the warps; the order is the same on every run.
+// A warp per binary took 104 us for one binary of a year (6000 tiles of 512 bins), this 22 us.
+constexpr int kReduceThreads = 256;
 __global__ void k_fused_reduce(const double* partials, const int* sup_start, const int* sup_len,
                                int B, int tile, double* d_h, double* h_h) {
-  const int lane = threadIdx.x & 31;
-  const int wpb = blockDim.x >> 5;
-  for (int b = blockIdx.x * wpb + (threadIdx.x >> 5); b < B; b += gridDim.x * wpb) {
-    double a = 0, c = 0, h = 0;
-    int s0 = sup_start[b], n = sup_len[b];
+  __shared__ double sums[kReduceThreads / 32][3];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int b = blockIdx.x; b < B; b += gridDim.x) {
+    double v[3] = {0.0, 0.0, 0.0};
+    const int s0 = sup_start[b], n = sup_len[b];
     if (n > 0) {
-      int tlo = s0 / tile, thi = (s0 + n - 1) / tile;
-      for (int t = tlo + lane; t <= thi; t += 32) {
+      const int tlo = s0 / tile, thi = (s0 + n - 1) / tile;
+      for (int t = tlo + threadIdx.x; t <= thi; t += kReduceThreads) {
         const double* P = partials + 3 * ((long long)t * B + b);
-        a += P[0];
-        c += P[1];
-        h += P[2];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) v[q] += P[q];
       }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      c += __shfl_xor_sync(0xffffffffu, c, o);
-      h += __shfl_xor_sync(0xffffffffu, h, o);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+      if (lane == 0) sums[warp][q] = v[q];
     }
-    if (lane == 0) {
-      d_h[2 * b] = 4.0 * a;
-      d_h[2 * b + 1] = 4.0 * c;
-      h_h[2 * b] = 4.0 * h;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        for (int w = 1; w < kReduceThreads / 32; ++w) v[q] += sums[w][q];
+      d_h[2 * b] = 4.0 * v[0];
+      d_h[2 * b + 1] = 4.0 * v[1];
+      h_h[2 * b] = 4.0 * v[2];
       h_h[2 * b + 1] = 0.0;
-      note_nonfinite(&g_nonfinite_likelihood, a, c, h, 0.0);
+      note_nonfinite(&g_nonfinite_likelihood, v[0], v[1], v[2], 0.0);
     }
+    __syncthreads();
   }
 }
 
@@ -1509,8 +1527,8 @@ int direct_fused_gh(cplx* gh, const long long* gh_off, double* d_h, double* h_h,
                   "k_direct_fused (d lnL / d h)");
   }
   if (!st && d_h != nullptr && h_h != nullptr) {
-    k_fused_reduce<<<grid_for(32LL * nb, 128), 128, 0, s>>>(part, start + b0, len + b0, nb, tile,
-                                                            d_h + 2LL * b0, h_h + 2LL * b0);
+    k_fused_reduce<<<grid_for(nb, 1), kReduceThreads, 0, s>>>(
+        part, start + b0, len + b0, nb, tile, d_h + 2LL * b0, h_h + 2LL * b0);
     st = launch_status("k_fused_reduce");
   }
   pool_free(part, s);
@@ -2077,8 +2095,8 @@ int bbhx_direct_like_fused(double* d_h, double* h_h, const double* data_freqs, c
     if (!st) st = launch_status("k_direct_fused");
   }
   if (!st) {
-    k_fused_reduce<<<grid_for(32LL * num_bin_all, 128), 128, 0, s>>>(part, sup, sup + num_bin_all,
-                                                                     num_bin_all, tile, d_h, h_h);
+    k_fused_reduce<<<grid_for(num_bin_all, 1), kReduceThreads, 0, s>>>(part, sup, sup + num_bin_all,
+                                                                       num_bin_all, tile, d_h, h_h);
     st = launch_status("k_fused_reduce");
   }
   pool_free(sup, s);

@@ -20,7 +20,7 @@ namespace bbhx {
 
 constexpr int SB_MAXGROUPS = 64;
 constexpr int SB_THREADS = 256;
-constexpr size_t kBuildSmemMax = 200 * 1024;
+constexpr size_t kBuildSmemMax = 204 * 1024;
 
 // One problem's build, in device memory (from bbhx_direct_source).
 struct BuildArgs {
@@ -31,7 +31,7 @@ struct BuildArgs {
   OrbitTables orb;
   double dspin, mf_min, mf_max, t_init, tL_start, tL_end, orb_tmin, orb_tmax;
   double *x, *y, *c1, *c2, *c3, *t_start, *t_end;
-  double* scratch;  // (4 + 9) L doubles per CTA when a row does not fit in shared memory
+  double* scratch;  // spline_work(L, 9) doubles per CTA when a row does not fit in shared memory
   ModeCoeffs* coeffs_out;  // heterodyned problems: the walkers' PhenomHM records (no build)
   int* flags;
   int nq, TDItag, rescaled, tdi2, run_phenomd, M, L, B;
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(SB_THREADS) k_sparse_build(const BuildMulti* _
     const long long r = row - H->roff[g];
     const int B = A.B, L = A.L;
     const int mm = A.run_phenomd ? 2 : A.mms[(int)(r % A.M)];
-    double* work = use_smem ? sb_smem : A.scratch + (size_t)blockIdx.x * (4 + 9) * H->max_length;
+    double* work = use_smem ? sb_smem : A.scratch + (size_t)blockIdx.x * spline_work(H->max_length, 9);
     {
       const unsigned long long* src = reinterpret_cast<const unsigned long long*>(recs + row);
       unsigned long long* dst = reinterpret_cast<unsigned long long*>(&R);
@@ -315,7 +315,7 @@ int bbhx_uneven_batch(const bbhx_direct_source* direct, int num_direct,
   int st = OK;
   std::vector<void*> scratch;
   if (H.ngroups > 0) {
-    const size_t smem = sizeof(double) * (size_t)(4 + 9) * maxL;
+    const size_t smem = sizeof(double) * spline_work(maxL, 9);
     const bool use_smem = smem <= kBuildSmemMax;
     const int nsm = sm_count();
     // two CTAs of SB_THREADS per SM (the register limit at 128 registers a thread)
@@ -328,7 +328,7 @@ int bbhx_uneven_batch(const bbhx_direct_source* direct, int num_direct,
     if (pool_alloc((void**)&dH, sizeof(BuildMulti), s) != cudaSuccess ||
         pool_alloc((void**)&recs, sizeof(RowRec) * (size_t)std::max(rows_direct, 1ll), s) != cudaSuccess ||
         pool_alloc((void**)&next, sizeof(unsigned long long), s) != cudaSuccess ||
-        (!use_smem && pool_alloc((void**)&work, sizeof(double) * grid * (size_t)(4 + 9) * maxL, s) != cudaSuccess)) {
+        (!use_smem && pool_alloc((void**)&work, sizeof(double) * grid * spline_work(maxL, 9), s) != cudaSuccess)) {
       set_error("device allocation for the sparse build failed");
       st = ERR_CUDA;
     }

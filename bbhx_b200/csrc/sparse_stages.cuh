@@ -216,23 +216,24 @@ __device__ __forceinline__ void phm_response_point(double* buf, long long n, lon
 
 // Not-a-knot spline of one system (knots xg[L], P quantities y[p * pstride + i]) by the whole
 // block: matrix once, P right-hand sides through one cyclic reduction in `work`
-// ((4 + P) L doubles: x, a, b, c, d[P][L]); slopes (optional) and c1, c2, c3 written in y's
+// (spline_work(L, P) doubles: a, b, c, w, d[P], permuted as cr_solve reads them); slopes (optional) and c1, c2, c3 written in y's
 // layout.  Entry L-1 of c1 / c2 / c3 holds the last row's (0, diagonal, lower) entries.
 // PT > 0 fixes P at compile time: a row's 3 PT (right-hand sides) and 2 PT (coefficients)
 // global loads are then issued together into registers instead of one quantity at a time.
+inline __host__ __device__ size_t spline_work(int L, int P) { return (size_t)(4 + P) * cr_pad(L); }
+
 template <int PT>
 __device__ inline void spline_system_t(const double* xg, const double* y, long long pstride,
                                        double* slopes, double* c1, double* c2, double* c3, int L,
                                        int Pr, double* work) {
   const int P = PT > 0 ? PT : Pr;
   constexpr int NV = PT > 0 ? PT : 1;
-  double* xs = work;
-  double* a = xs + L;
-  double* b = a + L;
-  double* c = b + L;
-  double* d = c + L;
-  for (int i = threadIdx.x; i < L; i += blockDim.x) xs[i] = xg[i];
-  __syncthreads();
+  const int ld = cr_pad(L);
+  double* a = work;
+  double* b = a + ld;
+  double* c = b + ld;
+  double* w = c + ld;
+  double* d = w + ld;
   for (int i = threadIdx.x; i < L; i += blockDim.x) {
     int i0, i1, i2;
     if (i == 0) {
@@ -242,15 +243,20 @@ __device__ inline void spline_system_t(const double* xg, const double* y, long l
     } else {
       i0 = i - 1; i1 = i; i2 = i + 1;
     }
-    const double dx1 = xs[i1] - xs[i0];
-    const double dx2 = xs[i2] - xs[i1];
-    const double dd = xs[i2] - xs[i0];
+    const double x0 = xg[i0], x1 = xg[i1], x2 = xg[i2];
+    const double dx1 = x1 - x0;
+    const double dx2 = x2 - x1;
+    const double dd = x2 - x0;
+    // reciprocals shared by the quantities: 18 divisions of a row become two
+    const double i1x = 1.0 / dx1, i2x = 1.0 / dx2;
+    const double idd = (i == 0 || i == L - 1) ? 1.0 / dd : 0.0;
+    const int j = cr_slot(i);
     if (i == 0) {
-      a[i] = 0.0; b[i] = dx2; c[i] = dd;
+      a[j] = 0.0; b[j] = dx2; c[j] = dd;
     } else if (i == L - 1) {
-      a[i] = dd; b[i] = dx1; c[i] = 0.0;
+      a[j] = dd; b[j] = dx1; c[j] = 0.0;
     } else {
-      a[i] = dx2; b[i] = 2 * (dx1 + dx2); c[i] = dx1;
+      a[j] = dx2; b[j] = 2 * (dx1 + dx2); c[j] = dx1;
     }
     for (int p0 = 0; p0 < P; p0 += NV) {
       double v0[NV], v1[NV], v2[NV];
@@ -263,27 +269,28 @@ __device__ inline void spline_system_t(const double* xg, const double* y, long l
       }
 #pragma unroll
       for (int q = 0; q < NV; ++q) {
-        const double m1 = (v1[q] - v0[q]) / dx1;
-        const double m2 = (v2[q] - v1[q]) / dx2;
+        const double m1 = (v1[q] - v0[q]) * i1x;
+        const double m2 = (v2[q] - v1[q]) * i2x;
         double r;
         if (i == 0)
-          r = ((dx1 + 2 * dd) * dx2 * m1 + dx1 * dx1 * m2) / dd;
+          r = ((dx1 + 2 * dd) * dx2 * m1 + dx1 * dx1 * m2) * idd;
         else if (i == L - 1)
-          r = (dx2 * dx2 * m1 + (2 * dd + dx2) * dx1 * m2) / dd;
+          r = (dx2 * dx2 * m1 + (2 * dd + dx2) * dx1 * m2) * idd;
         else
           r = 3.0 * (dx2 * m1 + dx1 * m2);
-        d[(size_t)(p0 + q) * L + i] = r;
+        d[(size_t)(p0 + q) * ld + j] = r;
       }
     }
   }
   __syncthreads();
   // keep the last row's matrix entries for the c1/c2/c3[L-1] convention
-  const double last_a = a[L - 1], last_b = b[L - 1];
+  const double last_a = a[cr_slot(L - 1)], last_b = b[cr_slot(L - 1)];
   __syncthreads();
-  cr_solve(a, b, c, d, L, P, L);
+  cr_solve(a, b, c, w, d, P, L);
   for (int i = threadIdx.x; i < L; i += blockDim.x) {
     const bool seg = i < L - 1;
-    const double h = seg ? xs[i + 1] - xs[i] : 1.0;
+    const double ih = seg ? 1.0 / (xg[i + 1] - xg[i]) : 1.0;
+    const int j = cr_slot(i), j1 = cr_slot(i + 1);
     for (int p0 = 0; p0 < P; p0 += NV) {
       double ylo[NV], yhi[NV];
 #pragma unroll
@@ -295,15 +302,15 @@ __device__ inline void spline_system_t(const double* xg, const double* y, long l
 #pragma unroll
       for (int q = 0; q < NV; ++q) {
         const long long o = (long long)(p0 + q) * pstride;
-        const double* sp = d + (size_t)(p0 + q) * L;
-        const double si = sp[i];
+        const double* sp = d + (size_t)(p0 + q) * ld;
+        const double si = sp[j];
         if (slopes) slopes[o + i] = si;
         if (seg) {
-          const double m = (yhi[q] - ylo[q]) / h;
-          const double t = (si + sp[i + 1] - 2 * m) / h;
+          const double m = (yhi[q] - ylo[q]) * ih;
+          const double t = (si + sp[j1] - 2 * m) * ih;
           c1[o + i] = si;
-          c2[o + i] = (m - si) / h - t;
-          c3[o + i] = t / h;
+          c2[o + i] = (m - si) * ih - t;
+          c3[o + i] = t * ih;
         } else {
           c1[o + i] = 0.0;
           c2[o + i] = last_b;

@@ -26,12 +26,12 @@ namespace bbhx {
 
 // x: [S, L]; y: [P, S, L]; outputs slopes / c1 / c2 / c3 in y's layout (any may alias the
 // reference's B / upper / diag / lower buffers).  `scratch` (used only when the system does
-// not fit in shared memory) holds gridDim.x * (4 + P) * L doubles.
+// not fit in shared memory) holds gridDim.x * spline_work(L, P) doubles.
 __global__ void k_spline(const double* __restrict__ x, const double* __restrict__ y,
                          double* slopes, double* c1, double* c2, double* c3, int L, int P,
                          long long S, bool use_smem, double* scratch) {
   extern __shared__ double smem[];
-  double* work = use_smem ? smem : scratch + (size_t)blockIdx.x * (4 + P) * L;
+  double* work = use_smem ? smem : scratch + (size_t)blockIdx.x * spline_work(L, P);
   for (long long sys = blockIdx.x; sys < S; sys += gridDim.x) {
     const long long o = sys * L;
     spline_system(x + o, y + o, S * L, slopes ? slopes + o : nullptr, c1 + o, c2 + o, c3 + o, L,
@@ -44,7 +44,7 @@ __global__ void k_spline(const double* __restrict__ x, const double* __restrict_
 using namespace bbhx;
 
 namespace {
-constexpr size_t kMaxSplineSmem = 200 * 1024;
+constexpr size_t kMaxSplineSmem = 204 * 1024;
 }
 
 extern "C" {
@@ -59,9 +59,9 @@ int bbhx_interpolate(const double* freqs, const double* y, double* B_, double* u
   long long S = (long long)num_modes * num_bin_all;
   if (S == 0) return OK;
   cudaStream_t s = (cudaStream_t)stream;
-  size_t smem = sizeof(double) * (size_t)(4 + num_interp_params) * length;
+  size_t smem = sizeof(double) * spline_work(length, num_interp_params);
   bool use_smem = smem <= kMaxSplineSmem;
-  int threads = 256;
+  int threads = 288;  // nine warps: one right-hand side each of the sparse buffer's nine
   const long long nsm = sm_count();
   unsigned int grid = (unsigned int)(S < nsm * 16 ? S : nsm * 16);
   double* scratch = nullptr;
@@ -70,7 +70,7 @@ int bbhx_interpolate(const double* freqs, const double* y, double* B_, double* u
                                          (int)kMaxSplineSmem));
   } else {
     grid = (unsigned int)(S < nsm * 2 ? S : nsm * 2);
-    BBHX_CHECK_CUDA(pool_alloc((void**)&scratch, sizeof(double) * grid * (4 + num_interp_params) * (size_t)length, s));
+    BBHX_CHECK_CUDA(pool_alloc((void**)&scratch, sizeof(double) * grid * spline_work(length, num_interp_params), s));
   }
   k_spline<<<grid, threads, use_smem ? smem : 0, s>>>(freqs, y, B_, upper_diag, diag, lower_diag,
                                                       length, num_interp_params, S, use_smem,

@@ -1,82 +1,100 @@
-// Block-cooperative tridiagonal solver shared by the spline build (spline.cu) and its
-// adjoint (gradient.cu).
+// Block-cooperative tridiagonal solver shared by the spline build (spline.cu, sparse_build.cu) and
+// its adjoint (gradient.cu).
 #pragma once
 
 #include "bbhx_common.cuh"
 
 namespace bbhx {
 
-// Forward-reduction step of cyclic reduction at stride s for row i = 2 s k + 2 s - 1.
-__device__ __forceinline__ void cr_reduce_row(double* a, double* b, double* c, double* d, int ld,
-                                              int P, int n, int s, int k) {
+// Cyclic reduction reads rows at strides of powers of two; every array is permuted within its groups
+// of 16 doubles (one bank cycle) so that such rows fall into different banks.
+__host__ __device__ __forceinline__ int cr_slot(int i) { return i ^ (((i >> 4) ^ (i >> 8)) & 15); }
+__host__ __device__ __forceinline__ int cr_pad(int n) { return (n + 15) & ~15; }  // length of an array
+
+// Forward step of cyclic reduction at stride s for row i = 2 s k + 2 s - 1: the matrix, whose two
+// multipliers go to w[2 k], w[2 k + 1] for the right-hand sides.
+__device__ __forceinline__ void cr_reduce_matrix(double* a, double* b, double* c, double* w, int n,
+                                                 int s, int k) {
   const int i = 2 * s * k + 2 * s - 1;
-  const int im = i - s, ip = i + s;
-  const bool hp = ip < n;
-  const double al = -a[i] / b[im];
-  const double ga = hp ? -c[i] / b[ip] : 0.0;
+  const int j = cr_slot(i), im = cr_slot(i - s);
+  const bool hp = i + s < n;
+  const int ip = hp ? cr_slot(i + s) : j;
+  const double al = -a[j] / b[im];
+  const double ga = hp ? -c[j] / b[ip] : 0.0;
   const double an = al * a[im];
-  const double bn = b[i] + al * c[im] + (hp ? ga * a[ip] : 0.0);
+  const double bn = b[j] + al * c[im] + (hp ? ga * a[ip] : 0.0);
   const double cn = hp ? ga * c[ip] : 0.0;
-  for (int p = 0; p < P; ++p) {
-    double* dp = d + (size_t)p * ld;
-    dp[i] = dp[i] + al * dp[im] + (hp ? ga * dp[ip] : 0.0);
-  }
-  a[i] = an;
-  b[i] = bn;
-  c[i] = cn;
+  a[j] = an;
+  b[j] = bn;
+  c[j] = cn;
+  w[2 * k] = al;
+  w[2 * k + 1] = ga;
+}
+__device__ __forceinline__ void cr_reduce_rhs(double* dp, const double* w, int n, int s, int k) {
+  const int i = 2 * s * k + 2 * s - 1;
+  const int j = cr_slot(i);
+  const double al = w[2 * k], ga = w[2 * k + 1];
+  const bool hp = i + s < n;
+  dp[j] = dp[j] + al * dp[cr_slot(i - s)] + (hp ? ga * dp[cr_slot(i + s)] : 0.0);
 }
 
-// Back-substitution step at stride s for row i = s - 1 + 2 s k (one division per row).
-__device__ __forceinline__ void cr_solve_row(const double* a, const double* b, const double* c,
-                                             double* d, int ld, int P, int n, int s, int k) {
-  const int i = s - 1 + 2 * s * k;
-  const int im = i - s, ip = i + s;
-  const double ib = 1.0 / b[i], ai = a[i], ci = c[i];
-  for (int p = 0; p < P; ++p) {
-    double* dp = d + (size_t)p * ld;
-    const double xm = (im >= 0) ? dp[im] : 0.0;
-    const double xp = (ip < n) ? dp[ip] : 0.0;
-    dp[i] = (dp[i] - ai * xm - ci * xp) * ib;
-  }
-}
-
-// In-place cyclic reduction on a[n], b[n], c[n] and P right-hand sides d[p*ld + i];
-// solution returned in d.  All threads of the block participate.  The levels with at most 32
-// active rows (the deep end of the reduction and the start of the substitution) run in warp 0
-// with warp-level synchronisation only, so the block meets at a barrier once per wide level.
-__device__ inline void cr_solve(double* a, double* b, double* c, double* d, int ld, int P, int n) {
-  const int t = threadIdx.x;
+// In-place cyclic reduction of P right-hand sides d[p * cr_pad(n) + cr_slot(i)] with the matrix
+// a, b, c (sub-diagonal, diagonal, super-diagonal, at cr_slot(i)); the solution returns in d, b is
+// replaced by its reciprocal.  w: cr_pad(n) doubles of scratch.  All threads of the block
+// participate.  The matrix is reduced once per level, by the block while a level has more than 32
+// rows, then by one warp; every warp takes right-hand sides of its own, and below the wide levels
+// runs them to the end with no barrier.  Bound by latency: 1024 knots x 9 quantities, one system 32
+// us, 6144 systems 1.30 ms (two blocks per SM); a row's thread walking all nine through conflicting
+// strides, and the levels of 32 rows or fewer left to one warp, took 55 us and 1.37 ms.
+__device__ inline void cr_solve(double* a, double* b, double* c, double* w, double* d, int P,
+                                int n) {
+  __shared__ double narrow[2 * 64];  // multipliers of the levels of 32 rows or fewer
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarp = (int)blockDim.x >> 5;
+  const int ld = cr_pad(n);
   int s = 1;
   for (; s < n && n / (2 * s) > 32; s <<= 1) {
     const int cnt = n / (2 * s);
-    for (int k = t; k < cnt; k += blockDim.x) cr_reduce_row(a, b, c, d, ld, P, n, s, k);
+    for (int k = t; k < cnt; k += blockDim.x) cr_reduce_matrix(a, b, c, w, n, s, k);
+    __syncthreads();
+    for (int p = warp; p < P; p += nwarp)
+      for (int k = lane; k < cnt; k += 32) cr_reduce_rhs(d + (size_t)p * ld, w, n, s, k);
     __syncthreads();
   }
-  if (t < 32) {
-    for (; s < n; s <<= 1) {
-      if (t < n / (2 * s)) cr_reduce_row(a, b, c, d, ld, P, n, s, t);
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  int top = 1;
+  const int s0 = s;
+  int top = s;
   while (top < n) top <<= 1;
-  auto count = [n](int st) { return (n >= st) ? (n - st) / (2 * st) + 1 : 0; };
-  s = top;
-  if (t < 32) {
-    for (; s >= 1 && count(s) <= 32; s >>= 1) {
-      if (t < count(s)) cr_solve_row(a, b, c, d, ld, P, n, s, t);
+  if (warp == 0) {
+    for (int r = s0, o = 0; r < n; r <<= 1) {
+      const int cnt = n / (2 * r);
+      if (lane < cnt) cr_reduce_matrix(a, b, c, narrow + 2 * o, n, r, lane);
+      o += cnt;
       __syncwarp();
     }
-  } else {
-    while (s >= 1 && count(s) <= 32) s >>= 1;
   }
   __syncthreads();
-  for (; s >= 1; s >>= 1) {
-    const int cnt = count(s);
-    for (int k = t; k < cnt; k += blockDim.x) cr_solve_row(a, b, c, d, ld, P, n, s, k);
-    __syncthreads();
+  for (int i = t; i < n; i += blockDim.x) b[cr_slot(i)] = 1.0 / b[cr_slot(i)];
+  __syncthreads();
+  for (int p = warp; p < P; p += nwarp) {
+    double* dp = d + (size_t)p * ld;
+    for (int r = s0, o = 0; r < n; r <<= 1) {
+      const int cnt = n / (2 * r);
+      if (lane < cnt) cr_reduce_rhs(dp, narrow + 2 * o, n, r, lane);
+      o += cnt;
+      __syncwarp();
+    }
+    for (int r = top; r >= 1; r >>= 1) {  // substitution, rows i = r - 1 + 2 r k
+      const int cnt = (n >= r) ? (n - r) / (2 * r) + 1 : 0;
+      for (int k = lane; k < cnt; k += 32) {
+        const int i = r - 1 + 2 * r * k;
+        const int j = cr_slot(i);
+        const double xm = (i - r >= 0) ? dp[cr_slot(i - r)] : 0.0;
+        const double xp = (i + r < n) ? dp[cr_slot(i + r)] : 0.0;
+        dp[j] = (dp[j] - a[j] * xm - c[j] * xp) * b[j];
+      }
+      __syncwarp();
+    }
   }
+  __syncthreads();
 }
 
 }  // namespace bbhx
