@@ -101,27 +101,6 @@ __device__ __forceinline__ int first_bin_at(double x, double xb, double k0, doub
   return i;
 }
 
-// Segment of f in the knots xr[0 .. L): searchsorted(right) - 1, guessed for the log-spaced knots
-// of the window regrid (per = (L - 1) / log(hi / lo)) and corrected, else by bisection.
-__device__ __forceinline__ int segment_guess(const double* __restrict__ xr, int L, double lo,
-                                             double hi, float per, double f) {
-  if (!(f >= lo)) return -1;
-  if (f >= hi) return L - 1;
-  int k = (int)(logf((float)(f / lo)) * per);
-  k = min(max(k, 0), L - 2);
-  for (int it = 0; it < 4; ++it) {
-    if (__ldg(xr + k) > f) k = max(k - 1, 0);
-    else if (__ldg(xr + k + 1) <= f) k = min(k + 1, L - 2);
-    else return k;
-  }
-  int a = 0, c = L;
-  while (a < c) {
-    const int mid = (a + c) >> 1;
-    if (__ldg(xr + mid) <= f) a = mid + 1; else c = mid;
-  }
-  return a - 1;
-}
-
 // Order-preserving integer of a float and back (warp max / min by integer reductions).
 __device__ __forceinline__ int order_key(float v) {
   const int b = __float_as_int(v);
@@ -296,44 +275,14 @@ __device__ __forceinline__ void panel_bins(const FusedArgs& A, const PanelStage&
   }
 }
 
-// What a panel walk does with the templates: sums <d|h>, <h|h> (kSum), the sums and d lnL / d h =
-// 4 w (d~ - w h) of every bin (kGrad), or the templates themselves (kTemplate).
-enum PanelMode { kSum, kGrad, kTemplate };
+template <bool GH>
+__device__ __forceinline__ void bin_products(const FusedArgs& A, cplx* gh, int i, const double* acc,
+                                             double& dr, double& di, double& hh);
 
-// Where the latter two go: bin i, channel c at p[i * bin + c * chan] (i counts data bins).
-struct PanelOut {
-  cplx* p;
-  long long bin, chan;
-};
-
-// One bin's template acc (6 reals): times weights and data into the sums, or written out.
-template <PanelMode MODE>
-__device__ __forceinline__ void bin_products(const FusedArgs& A, const PanelOut& out, int i,
-                                             const double* acc, double& dr, double& di, double& hh) {
-  if (MODE == kTemplate) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) out.p[i * out.bin + c * out.chan] = mk(acc[2 * c], acc[2 * c + 1]);
-    return;
-  }
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    const long long gi = (long long)c * A.N + i;
-    const double w = __ldg(A.noise + gi);
-    const double2 d = __ldg(reinterpret_cast<const double2*>(A.data) + gi);
-    const double hr = acc[2 * c] * w, hi = acc[2 * c + 1] * w;
-    dr = fma(d.x, hr, fma(d.y, hi, dr));
-    di = fma(d.x, hi, fma(-d.y, hr, di));
-    hh = fma(hr, hr, fma(hi, hi, hh));
-    if (MODE == kGrad)
-      out.p[i * out.bin + c * out.chan] = mk(4.0 * w * (d.x - hr), 4.0 * w * (d.y - hi));
-  }
-}
-
-// panel_bins where the template of every bin is needed: with the carrier e^{i b (i - ia)} bin by
-// bin (rotated along the lane's bins).
-template <PanelMode MODE>
-__device__ __forceinline__ void panel_bins_out(const FusedArgs& A, const PanelOut& out,
-                                              const PanelStage& PS, int ia, int n, double center, double inv_half,
+// panel_bins for the gradient: the same sums and d lnL / d h = 4 w (d~ - w h) of every bin, which
+// needs the carrier e^{i b (i - ia)} bin by bin (rotated along the lane's bins).
+__device__ __forceinline__ void panel_bins_gh(const FusedArgs& A, cplx* gh, const PanelStage& PS,
+                                              int ia, int n, double center, double inv_half,
                                               int lane, double Rr, double Ri, double& dr,
                                               double& di, double& hh) {
   const double s0 = ((double)lane - center) * inv_half, ds = 32.0 * inv_half;
@@ -372,21 +321,38 @@ __device__ __forceinline__ void panel_bins_out(const FusedArgs& A, const PanelOu
         f[t][2 * ch + 1] = -fma(qr[t], ci[t], qi[t] * cr[t]);
       }
     }
-    bin_products<MODE>(A, out, ia + i, f[0], dr, di, hh);
-    if (i + 32 < n) bin_products<MODE>(A, out, ia + i + 32, f[1], dr, di, hh);
+    bin_products<true>(A, gh, ia + i, f[0], dr, di, hh);
+    if (i + 32 < n) bin_products<true>(A, gh, ia + i + 32, f[1], dr, di, hh);
+  }
+}
+
+// One bin's template acc (6 reals) times weights and data, into the sums; GH: and its d lnL / d h =
+// 4 w (d~ - w h) to gh[3 i + channel] (gh addressed by data bin).
+template <bool GH>
+__device__ __forceinline__ void bin_products(const FusedArgs& A, cplx* gh, int i, const double* acc,
+                                             double& dr, double& di, double& hh) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const long long gi = (long long)c * A.N + i;
+    const double w = __ldg(A.noise + gi);
+    const double2 d = __ldg(reinterpret_cast<const double2*>(A.data) + gi);
+    const double hr = acc[2 * c] * w, hi = acc[2 * c + 1] * w;
+    dr = fma(d.x, hr, fma(d.y, hi, dr));
+    di = fma(d.x, hi, fma(-d.y, hr, di));
+    hh = fma(hr, hr, fma(hi, hi, hh));
+    if (GH) gh[3LL * i + c] = mk(4.0 * w * (d.x - hr), 4.0 * w * (d.y - hi));
   }
 }
 
 // The n bins from ia one by one (lanes over bins) where the knots lie as close as the bins: every
-// bin finds its own segment of each mode and reads the spline arrays (freqs: the grid, if it is
-// not k df).
-template <PanelMode MODE>
-__device__ __forceinline__ void panel_scatter(const FusedArgs& A, const PanelOut& out,
-                                              const PanelStage& PS, int b, int ia, int n, int lane, double k0, double df,
+// bin finds its own segment of each mode and reads the spline arrays.
+template <bool GH>
+__device__ __forceinline__ void panel_scatter(const FusedArgs& A, cplx* gh, const PanelStage& PS,
+                                              int b, int ia, int n, int lane, double k0, double df,
                                               double ts, double te, double& dr, double& di,
-                                              double& hh, const double* freqs = nullptr) {
+                                              double& hh) {
   for (int i = ia + lane; i < ia + n; i += 32) {
-    const double f = freqs ? __ldg(freqs + i) : __dmul_rn(k0 + (double)i, df);
+    const double f = __dmul_rn(k0 + (double)i, df);
     double acc[6] = {0, 0, 0, 0, 0, 0};
     for (int m = 0; m < A.M; ++m) {
       const long long o = ((long long)b * A.M + m) * A.L;
@@ -394,16 +360,15 @@ __device__ __forceinline__ void panel_scatter(const FusedArgs& A, const PanelOut
       if (k >= 0 && k < A.L - 1)
         accumulate_bin_src(GlobalCoef{A, o + k, __ldg(A.x + o + k)}, f, ts, te, acc);
     }
-    bin_products<MODE>(A, out, i, acc, dr, di, hh);
+    bin_products<GH>(A, gh, i, acc, dr, di, hh);
   }
 }
 
 // The n bins from ia one by one, G bins per lane at a time: runs where a mode crosses the
 // observation window (GATE: its t(f) decides bin by bin) or the modes' phases do not stay
 // together.
-template <int G, bool GATE, PanelMode MODE>
-__device__ __forceinline__ void panel_direct(const FusedArgs& A, const PanelOut& out,
-                                             const PanelStage& PS, int b,
+template <int G, bool GATE, bool GH>
+__device__ __forceinline__ void panel_direct(const FusedArgs& A, cplx* gh, const PanelStage& PS, int b,
                                              int ia, int n, int lane, double k0, double df,
                                              double& dr, double& di, double& hh) {
   double ts = 0.0, te = 0.0;
@@ -465,7 +430,7 @@ __device__ __forceinline__ void panel_direct(const FusedArgs& A, const PanelOut&
     }
 #pragma unroll
     for (int j = 0; j < G; ++j)
-      if (i + 32 * j < n) bin_products<MODE>(A, out, ia + i + 32 * j, acc[j], dr, di, hh);
+      if (i + 32 * j < n) bin_products<GH>(A, gh, ia + i + 32 * j, acc[j], dr, di, hh);
   }
   __syncwarp();
 }
@@ -473,14 +438,15 @@ __device__ __forceinline__ void panel_direct(const FusedArgs& A, const PanelOut&
 // Bins [i0, i1) of binary b (inside its support) by one warp; kk = the segments of bins i0 and
 // i1 - 1 in lanes 0 .. M-1 (-1 before a mode's first knot, L-1 past its last).  Lane m walks mode
 // m.  When a mode enters segment k its freed ring slot is refilled with segment k + 3 by
-// asynchronous copies, three entries ahead of their use.  Per-lane partial sums into dr, di, hh
-// and what MODE asks for into out.
-template <PanelMode MODE>
+// asynchronous copies, three entries ahead of their use.  Per-lane partial sums into dr, di, hh;
+// GH: also d lnL / d h of every bin to A.gh (gradient chain).
+template <bool GH>
 __device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, int b, int i0,
                                            int i1, int2 kk, int lane, double k0, double df,
-                                           double& dr, double& di, double& hh,
-                                           const PanelOut& out = PanelOut{nullptr, 0, 0}) {
+                                           double& dr, double& di, double& hh) {
   const int M = A.M, L = A.L;
+  cplx* gh = nullptr;
+  if (GH) gh = A.gh + 3 * (__ldg(A.gh_off + b) - (long long)__ldg(A.sup_start + b));
   const bool mine = lane < M;
   int k = mine ? kk.x : L - 1;
   const int klast = mine ? min(kk.y, L - 2) : -1;  // last segment of the item
@@ -505,7 +471,7 @@ __device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, i
       dens = __shfl_sync(0xffffffffu, dens, 0);
       if (!(dens * (float)kPanelMinBins > 1.0f)) break;
       const int n = min(kPanelDirect, i1 - i);
-      panel_scatter<MODE>(A, out, PS, b, i, n, lane, k0, df, ts, te, dr, di, hh);
+      panel_scatter<GH>(A, gh, PS, b, i, n, lane, k0, df, ts, te, dr, di, hh);
       i += n;
       if (i >= i1) return;
       if (mine) k = segment_guess(xr, L, lo, hi, per, __dmul_rn(k0 + (double)i, df));
@@ -596,13 +562,12 @@ __device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, i
     int n = e - i;
     const unsigned act = __ballot_sync(0xffffffffu, gate != 2);
     if (act == 0u) {
-      if (MODE != kSum)
-        panel_direct<1, false, MODE>(A, out, PS, b, i, n, lane, k0, df, dr, di, hh);  // h = 0
+      if (GH) panel_direct<1, false, GH>(A, gh, PS, b, i, n, lane, k0, df, dr, di, hh);  // h = 0
       i = e;
       continue;
     }
     if (__any_sync(0xffffffffu, gate == 0)) {
-      panel_direct<1, true, MODE>(A, out, PS, b, i, n, lane, k0, df, dr, di, hh);
+      panel_direct<1, true, GH>(A, gh, PS, b, i, n, lane, k0, df, dr, di, hh);
       i = e;
       continue;
     }
@@ -625,7 +590,7 @@ __device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, i
       const float fit = n * fminf(1.0f, fminf(kPanelDelta / lin, sqrtf(kPanelQuad / quad)));
       if (!(fit >= (float)kPanelMinBins)) {
         n = min(n, kPanelDirect);
-        panel_direct<2, false, MODE>(A, out, PS, b, i, n, lane, k0, df, dr, di, hh);
+        panel_direct<2, false, GH>(A, gh, PS, b, i, n, lane, k0, df, dr, di, hh);
         i += n;
         continue;
       }
@@ -651,12 +616,12 @@ __device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, i
       cap = n;
     }
     if (!smooth) {
-      panel_direct<2, false, MODE>(A, out, PS, b, i, n, lane, k0, df, dr, di, hh);
+      panel_direct<2, false, GH>(A, gh, PS, b, i, n, lane, k0, df, dr, di, hh);
       i += n;
       continue;
     }
-    if constexpr (MODE != kSum) {
-      panel_bins_out<MODE>(A, out, PS, i, n, center, 1.0 / half, lane, Rr, Ri, dr, di, hh);
+    if constexpr (GH) {
+      panel_bins_gh(A, gh, PS, i, n, center, 1.0 / half, lane, Rr, Ri, dr, di, hh);
     } else {
       double zr, zi;
       panel_bins(A, PS, i, n, center, 1.0 / half, lane, Rr, Ri, zr, zi, hh);

@@ -791,7 +791,7 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
       if (uni) {
         const int2 kk = (lane < A.M) ? A.segtab[q * A.M + lane] : make_int2(0, 0);
         double dr = 0.0, di = 0.0, hh = 0.0;
-        panel_item<kSum>(A, *PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, gk0, gdf, dr, di,
+        panel_item<false>(A, *PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, gk0, gdf, dr, di,
                           hh);
         for (int o = 16; o > 0; o >>= 1) {
           dr += __shfl_xor_sync(0xffffffffu, dr, o);
@@ -1175,10 +1175,7 @@ __global__ void __launch_bounds__(FD_WARPS * 32, 3) k_direct_panel(FusedArgs A) 
     double dr = 0.0, di = 0.0, hh = 0.0;
     if (t0 < s1 && t0 + A.tile > s0) {
       const int2 kk = (lane < A.M) ? A.segtab[q * A.M + lane] : make_int2(0, 0);
-      PanelOut out{nullptr, 3, 1};
-      if (GH) out.p = A.gh + 3 * (__ldg(A.gh_off + b) - (long long)s0);
-      panel_item<GH ? kGrad : kSum>(A, PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, k0, df,
-                                    dr, di, hh, out);
+      panel_item<GH>(A, PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, k0, df, dr, di, hh);
       for (int o = 16; o > 0; o >>= 1) {
         dr += __shfl_xor_sync(0xffffffffu, dr, o);
         di += __shfl_xor_sync(0xffffffffu, di, o);
@@ -1192,42 +1189,6 @@ __global__ void __launch_bounds__(FD_WARPS * 32, 3) k_direct_panel(FusedArgs A) 
       P[2] = hh;
     }
     __syncwarp();
-  }
-}
-
-// Templates of the binaries on the data grid (TemplateInterpFD, waveformbuild.py:89-239), all bins
-// of each support: panels on uniform grids, else bin by bin with each bin's own segment search.
-// tmpl [B]: [3, len] arrays.
-__global__ void __launch_bounds__(FD_WARPS * 32, 3) k_templates(FusedArgs A, cplx* const* tmpl) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const unsigned ok = A.grid->ok & 7u;
-  const int lane = threadIdx.x & 31;
-  PanelStage& PS = reinterpret_cast<PanelStage*>(smem_raw)[threadIdx.x >> 5];
-  const double k0 = A.grid->k0, df = A.grid->df[(ok & 1u) ? 0 : (ok & 2u) ? 1 : 2];
-  const long long nitems = (long long)A.ntiles * A.B;
-  for (long long q = claim_item(A.next, lane); q < nitems; q = claim_item(A.next, lane)) {
-    const int tile = (int)(q / A.B);
-    const int b = (int)(q - (long long)tile * A.B);
-    const int s0 = __ldg(A.sup_start + b), len = __ldg(A.sup_len + b), s1 = s0 + len;
-    const int i0 = max(tile * A.tile, s0), i1 = min((tile + 1) * A.tile, s1);
-    if (i0 >= i1) continue;
-    const PanelOut out{tmpl[b] - s0, 1, len};
-    double none[3];
-    if (ok) {
-      const int2 kk = (lane < A.M) ? A.segtab[q * A.M + lane] : make_int2(0, 0);
-      panel_item<kTemplate>(A, PS, b, i0, i1, kk, lane, k0, df, none[0], none[1], none[2], out);
-    } else {
-      if (lane < A.M) {
-        const double* xr = A.x + ((long long)b * A.M + lane) * A.L;
-        PS.lo[lane] = __ldg(xr);
-        PS.hi[lane] = __ldg(xr + A.L - 1);
-        PS.per[lane] = (float)(A.L - 1) / logf((float)(PS.hi[lane] / PS.lo[lane]));
-      }
-      __syncwarp();
-      panel_scatter<kTemplate>(A, out, PS, b, i0, i1 - i0, lane, k0, df, __ldg(A.t_start + b),
-                               __ldg(A.t_end + b), none[0], none[1], none[2], A.data_freqs);
-      __syncwarp();
-    }
   }
 }
 
@@ -1631,97 +1592,6 @@ int bbhx_selftest_recurrence(const double* pc, double xk, double k0, double df, 
   k_selftest_recurrence<<<(lanes + 127) / 128, 128, 0, (cudaStream_t)stream>>>(pc, xk, k0, df,
                                                                               lanes, steps, out);
   return launch_status("k_selftest_recurrence");
-}
-
-// Templates of num_bin_all binaries on the data grid from their splines, all bins of each support
-// (the reference's InterpTDI without its index arrays): template_ptrs (device addresses of
-// [3, lengths[b]] complex128 arrays), t_start, t_end, starts, lengths are HOST arrays; num_modes
-// 1..6.
-int bbhx_interp_templates(const int64_t* template_ptrs, const double* data_freqs, const double* x,
-                          const double* y, const double* c1, const double* c2, const double* c3,
-                          const double* t_start, const double* t_end, int length, int data_length,
-                          int num_bin_all, int num_modes, const int* starts, const int* lengths,
-                          void* stream) {
-  BBHX_REQUIRE(length >= 2 && num_modes >= 1 && num_modes <= FD_MAXM && data_length >= 1, "bad sizes");
-  if (num_bin_all == 0) return OK;
-  cudaStream_t s = (cudaStream_t)stream;
-  const int B = num_bin_all, M = num_modes;
-  // template addresses, observation limits, supports: one block, one copy
-  const size_t words = (size_t)B * 4;
-  std::vector<uint64_t> host(words);
-  int* hs = reinterpret_cast<int*>(host.data() + 3 * (size_t)B);
-  for (int b = 0; b < B; ++b) {
-    BBHX_REQUIRE(lengths[b] >= 0 && starts[b] >= 0 &&
-                     (long long)starts[b] + lengths[b] <= data_length,
-                 "binary %d: data range [%d, %d) outside the data grid", b, starts[b],
-                 starts[b] + lengths[b]);
-    host[b] = (uint64_t)template_ptrs[b];
-    memcpy(&host[B + (size_t)b], &t_start[b], 8);
-    memcpy(&host[2 * (size_t)B + b], &t_end[b], 8);
-    hs[b] = starts[b];
-    hs[B + b] = lengths[b];
-  }
-  const int tile = fused_tile(data_length, B, FD_TILE);
-  const int ntiles = (data_length + tile - 1) / tile;
-  const long long nitems = (long long)ntiles * B;
-  uint64_t* dev = nullptr;
-  int2* segtab = nullptr;
-  GridInfo* grid = nullptr;
-  unsigned long long* next = nullptr;
-  BBHX_CHECK_CUDA(pool_alloc_all(s, {{(void**)&dev, 8 * words},
-                                     {(void**)&segtab, sizeof(int2) * nitems * M},
-                                     {(void**)&grid, sizeof(GridInfo)},
-                                     {(void**)&next, sizeof(unsigned long long)}}));
-  int st = cuda_status(cudaMemcpyAsync(dev, host.data(), 8 * words, cudaMemcpyHostToDevice, s),
-                       "template job upload");
-  const int* sup = reinterpret_cast<const int*>(dev + 3 * (size_t)B);
-  if (!st) st = detect_grid(data_freqs, data_length, grid, s);
-  if (!st) {
-    k_tile_segments<<<grid_for(nitems * M, 256, sm_count() * 64), 256, 0, s>>>(
-        segtab, x, data_freqs, sup, sup + B, B, M, length, ntiles, tile);
-    st = launch_status("k_tile_segments");
-  }
-  if (!st)
-    st = cuda_status(cudaMemsetAsync(next, 0, sizeof(unsigned long long), s), "work-queue counter");
-  const size_t sm = FD_WARPS * sizeof(PanelStage);
-  if (!st)
-    st = cuda_status(cudaFuncSetAttribute(k_templates, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)sm),
-                     "cudaFuncSetAttribute(k_templates)");
-  if (!st) {
-    FusedArgs A;
-    memset(&A, 0, sizeof(A));
-    A.data_freqs = data_freqs;
-    A.N = data_length;
-    A.x = x;
-    A.y = y;
-    A.c1 = c1;
-    A.c2 = c2;
-    A.c3 = c3;
-    A.t_start = reinterpret_cast<const double*>(dev + B);
-    A.t_end = reinterpret_cast<const double*>(dev + 2 * (size_t)B);
-    A.sup_start = sup;
-    A.sup_len = sup + B;
-    A.B = B;
-    A.M = M;
-    A.L = length;
-    A.ntiles = ntiles;
-    A.tile = tile;
-    A.segtab = segtab;
-    A.qstride = (long long)B * M * length;
-    A.grid = grid;
-    A.next = next;
-    k_templates<<<resident_grid(k_templates, sm, nitems), FD_WARPS * 32, sm, s>>>(
-        A, reinterpret_cast<cplx* const*>(dev));
-    st = launch_status("k_templates");
-  }
-  pool_free(dev, s);
-  pool_free(segtab, s);
-  pool_free(grid, s);
-  pool_free(next, s);
-  // the host block must outlive the copy
-  const cudaError_t e = cudaStreamSynchronize(s);
-  return st ? st : cuda_status(e, "template sync");
 }
 
 // Support [start, start+len) of each binary on the data grid (device int arrays).

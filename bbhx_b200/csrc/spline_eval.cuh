@@ -38,6 +38,27 @@ __device__ __forceinline__ void combine_channels(double amp, double phase, cplx 
   h3 = conj(T3 * ap);
 }
 
+// Segment of f in the knots xr[0 .. L): searchsorted(right) - 1, guessed for the log-spaced knots
+// of the window regrid (per = (L - 1) / log(hi / lo)) and corrected, else by bisection.
+__device__ __forceinline__ int segment_guess(const double* __restrict__ xr, int L, double lo,
+                                             double hi, float per, double f) {
+  if (!(f >= lo)) return -1;
+  if (f >= hi) return L - 1;
+  int k = (int)(logf((float)(f / lo)) * per);
+  k = min(max(k, 0), L - 2);
+  for (int it = 0; it < 4; ++it) {
+    if (__ldg(xr + k) > f) k = max(k - 1, 0);
+    else if (__ldg(xr + k + 1) <= f) k = min(k + 1, L - 2);
+    else return k;
+  }
+  int a = 0, c = L;
+  while (a < c) {
+    const int mid = (a + c) >> 1;
+    if (__ldg(xr + mid) <= f) a = mid + 1; else c = mid;
+  }
+  return a - 1;
+}
+
 // warp-cooperative searchsorted(row, v, side='right') - 1 over a sorted row of length L;
 // every lane passes the same v and receives the same result in [-1, L-1].
 __device__ __forceinline__ int warp_segment_search(const double* __restrict__ row, int L, double v) {

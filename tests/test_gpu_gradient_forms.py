@@ -2,8 +2,9 @@
 options where it branches: point counts around a warp's 32 and around the split of a (binary, mode)
 over several warps, one mode and six, XYZ and AET, both TDI generations, and a source along an arm
 (the series form of 1 / (1 - k.n)).  Oracle: central finite differences of the FP64 lnL with the
-steps of tests/test_gpu_gradient.py and twice them, without the h^2 term (the phase moves by 0.1 rad
-per step in some spins: that term alone is 2e-4 there; halved steps would double the rounding noise), and its bound (1e-4 relative plus
+steps of tests/test_gpu_gradient.py (ten times them for the angles, whose phases move least, against
+the rounding of lnL over the step) and twice those, without the h^2 term (the phase moves by 0.1 rad
+per step in some spins: that term alone is 2e-4 there), and its bound (1e-4 relative plus
 1e-7 of the largest scaled component)."""
 import numpy as np
 import pytest
@@ -17,6 +18,7 @@ def _extrapolated_fd(fn, P):
     """fn: [12, B] -> lnL [B]; returns [B, 11] central differences without their h^2 term."""
     B = P.shape[1]
     steps = np.array([_steps(P[:, b]) for b in range(B)])
+    steps[:, 5:10] *= 10.0  # phi_ref, inc, lam, beta, psi
     out = np.zeros((B, len(ROWS)))
     for k, r in enumerate(ROWS):
         fd = []
