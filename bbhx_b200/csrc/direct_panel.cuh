@@ -12,7 +12,7 @@
 // instructions per bin for six modes with everything included, against 306.  Where the modes do
 // not stay together (1-4 % of the band of a 1-yr stream) the bins are evaluated one by one.
 //
-// What bounds it (B = 1024, 1 yr, six modes, L = 1024; 86.4 ms before the panels, 26 ms now): the
+// What bounds it (B = 1024, 1 yr, six modes, L = 1024; 86.4 ms before the panels, 27 ms now): the
 // FP64 pipe is 50 % busy counted at 2 cycles an instruction, but a DFMA that reads three
 // registers anew takes 3 (40.7 of 64 lanes per clock measured, 53 in the order of panel_bins), so
 // the pipe is two thirds busy, the shared-memory and load path 60 %, issue 50 %.  Data in L1

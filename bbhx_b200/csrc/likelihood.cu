@@ -1410,8 +1410,8 @@ unsigned resident_grid(K kernel, size_t smem, long long nitems) {
 
 // Data bins per work item of a single-problem launch: the largest tile up to `tile` that still
 // gives every resident warp several items, since an item of a low-frequency tile takes many times
-// the average and the call ends when its slowest item does (B = 1, 1 yr: 1.03 ms at 4096 bins,
-// 0.25 ms at 512; B = 1024: 1.1 ms less at 8192 bins than at 4096).
+// the average and the call ends when its slowest item does (call with B = 1, 1 yr: 1.81 ms at 4096
+// bins, 0.86 ms at 512; B = 1024: 1.1 ms less at 8192 bins than at 4096).
 inline int fused_tile(int N, int B, int tile) {
   const long long warps = (long long)sm_count() * 3 * FD_WARPS;
   while (tile > 256 && ((long long)N + tile - 1) / tile * B < 8 * warps) tile >>= 1;

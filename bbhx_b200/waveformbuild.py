@@ -85,7 +85,7 @@ class TemplateInterpFD:
 
     def _templates(self, data_freqs, freqs, y, c1, c2, c3, ts, te):
         """The same templates by bbhx_interp_templates, which finds the bins' segments itself (the
-        index arrays and their searches took 40 % of an injection)."""
+        index arrays and their searches took half of an injection)."""
         t = torch()
         B, M, L = self.num_bin_all, self.num_modes, self.length
         sup = t.empty(2 * B, dtype=t.int32, device=device())

@@ -41,15 +41,16 @@ SEED_PARAMS = 1234
 SEED_NOISE = 99
 HBM_BYTES_PER_PAIR = 72.0  # 3 x complex128 weighted data + 3 x float64 noise weights
 MIXED_BYTES_PER_PAIR = 36.0  # 3 x complex64 + 3 x float32: the FP32 copies the mixed form reads
-# FP64 instructions per (pair, mode) the direct algorithm cannot do without: 7 cubics (amplitude,
-# 3 complex transfer functions) x 3 FMAs, 3 complex products of the phase recurrence x 4, the
-# amplitude times e^{i phi} 2, and the 3 channels' complex multiply-accumulates x 4
-FP64_INSTR_PER_PAIR_MODE = 7 * 3 + 3 * 4 + 2 + 3 * 4
+# FP64 instructions per (binary, bin) pair the panel form cannot do without, whatever the number of
+# modes: per channel a complex polynomial of degree 7 (14), the carrier product (4), and the products
+# with weight and data (8)
+FP64_INSTR_PER_PAIR = 3 * (14 + 4 + 8)
 # the library's kernels in one direct step (ncu launch list): k_clear_flags, k_step_front,
 # k_ringdown_hm, k_ringdown_d, k_phm_setup, k_default_freqs, k_phm_tf, k_tf_window,
 # k_response_setup, k_phm_response, k_tf_range, k_spline, k_support, k_grid_detect,
-# k_tile_segments, k_direct_fused, k_fused_reduce, k_pack_lnl
-LAUNCHES_PER_STEP = 18
+# k_tile_segments, k_direct_panel, k_direct_fused (returns at once on uniform grids),
+# k_fused_reduce, k_pack_lnl
+LAUNCHES_PER_STEP = 19
 
 
 def parse():
@@ -419,10 +420,10 @@ def gpu_arm(args):
                      "frac": achieved / peak,
                      "algorithmic_bytes_per_pair": HBM_BYTES_PER_PAIR,
                      "traffic": (tpp * pairs if tpp is not None else None),
-                     "kernel": "k_direct_fused<FP64> (bbhx_direct_like_fused, precision 0)",
+                     "kernel": "k_direct_panel (bbhx_direct_like_fused, precision 0)",
                      "kernel_ms": statistics.mean(fused_ms),
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback",
-                     "fp64_floor": fp64_floor(pairs, wave.num_modes, fused_avg_s, peak)},
+                     "fp64_floor": fp64_floor(pairs, fused_avg_s, peak)},
         "gpu_launches": LAUNCHES_PER_STEP * args.steps,
         "clocks": clocks,
     }
@@ -569,13 +570,13 @@ OPC_NAMES = ("add_sub", "mul", "div", "compare", "sqrt", "cbrt", "log", "exp", "
              "sin_cos", "other")
 
 
-def fp64_floor(pairs, modes, kernel_s, hbm_peak_gbs):
-    """The FP64 pipe's bound on the direct kernel: FP64_INSTR_PER_PAIR_MODE instructions for every
-    (pair, mode) (pairs x modes is an upper bound: every mode counted over the union support) at
-    the nominal FP64 lane rate give the shortest possible kernel time, and the HBM-roofline
-    fraction the kernel would reach there."""
-    floor_s = FP64_INSTR_PER_PAIR_MODE * pairs * modes / fp64_lane_rate()
-    return {"fp64_instr_per_pair_mode": FP64_INSTR_PER_PAIR_MODE, "floor_ms": floor_s * 1e3,
+def fp64_floor(pairs, kernel_s, hbm_peak_gbs):
+    """The FP64 pipe's bound on the direct kernel: FP64_INSTR_PER_PAIR instructions for every pair
+    (the panels' nodes and the bins evaluated one by one come on top) at the nominal FP64 lane rate
+    give the shortest possible kernel time, and the HBM-roofline fraction the kernel would reach
+    there."""
+    floor_s = FP64_INSTR_PER_PAIR * pairs / fp64_lane_rate()
+    return {"fp64_instr_per_pair": FP64_INSTR_PER_PAIR, "floor_ms": floor_s * 1e3,
             "kernel_over_floor": kernel_s / floor_s,
             "hbm_frac_at_floor": HBM_BYTES_PER_PAIR * pairs / floor_s / 1e9 / hbm_peak_gbs,
             "lane_rate": "the device's SMs x 64 FP64 lanes x 1965 MHz (nominal clock)"}
@@ -799,7 +800,10 @@ def cpu_baseline(args):
     CPU_WARMUP.  Also the single-thread "as shipped" figure: the reference's CPU build never
     enables OpenMP, so one binary on one core is what its own build delivers."""
     from bbhx_b200.synthetic import draw_params
+    from oracle.build_ref import OUT
 
+    if not os.path.exists(OUT):
+        return {"unavailable": "the reference's CPU library is not built (oracle/build_ref.py)"}
     params = draw_params(args.batch, TOBS, SEED_PARAMS)
     workers = cpu_workers()
     val, times = cpu_reference(params, workers, steps=CPU_STEPS, warmup=CPU_WARMUP)
