@@ -250,6 +250,8 @@ struct FusedArgs {
   int B, M, L;
   int ntiles;
   int tile;            // data bins per tile item (multiple of FD_WARP_BINS)
+  int block;           // mixed form: bins (a multiple of tile) whose segment counts choose the
+                       // FP32 arithmetic (fused_item)
   double* partials;    // [ntiles * B][3]
   const int2* segtab;  // [ntiles][B][M]: segments of the tile's first and last bin
   double* d_h;         // [B] complex outputs
@@ -753,6 +755,10 @@ namespace bbhx {
 // block-wide barrier is involved.  Modes whose tile spans more than NSEG segments (low
 // frequencies) are staged a window of NSEG segments at a time from a forward cursor in the FP64
 // form, and walked per lane over global memory in the mixed form.
+// The mixed form rounds a (bin, mode) differently in a staged segment (accumulate_chunk,
+// accumulate_group) and on the walk (accumulate_bin), so which one it takes must not follow the
+// item's size, which fused_tile chooses by the number of binaries in the call: it is decided by
+// the segments of the aligned A.block bins around the item.
 // MIXED: phase, t(f), the phase reduction and all accumulations in FP64; amplitude, transfer
 // functions, sin/cos of the reduced phase and the mode sum (the template) in FP32; the per-bin
 // products with data and weights in FP64 when the FP32 copies of data and weights are given
@@ -813,8 +819,16 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
       const int2 kk = A.segtab[q * A.M + lane];
       const int klo = max(kk.x, 0), khi = min(kk.y, L - 2);
       const int n = (kk.x > kk.y || khi < klo) ? 0 : khi - klo + 1;
+      bool many = n > WarpStage<R>::NSEG;
+      if (MIXED && A.block > A.tile) {
+        const int k0 = (t0 / A.block) * A.block;
+        const int ta = max(k0, s0) / A.tile, tz = (min(k0 + A.block, s1) - 1) / A.tile;
+        const int ka = A.segtab[((long long)ta * A.B + b) * A.M + lane].x;
+        const int kz = A.segtab[((long long)tz * A.B + b) * A.M + lane].y;
+        many = min(kz, L - 2) - max(ka, 0) + 1 > WarpStage<R>::NSEG;
+      }
       S.klo[lane] = klo;
-      S.nseg[lane] = (n > WarpStage<R>::NSEG) ? -1 : n;
+      S.nseg[lane] = (n > 0 && many) ? -1 : n;
       S.kcur[lane] = klo;
       S.nst[lane] = 0;
     }
@@ -1461,6 +1475,7 @@ int direct_fused_gh(cplx* gh, const long long* gh_off, double* d_h, double* h_h,
     A.L = L;
     A.ntiles = ntiles;
     A.tile = tile;
+    A.block = tile;
     A.partials = part;
     A.segtab = segtab;
     A.d_h = nullptr;
@@ -1716,6 +1731,7 @@ int uneven_like(const bbhx_direct_group* groups, int num_groups,
     A.M = G.num_modes;
     A.L = G.length;
     A.tile = tile_bins;
+    A.block = tile_bins;
     A.ntiles = (G.data_length + tile_bins - 1) / tile_bins;
     A.d_h = (double*)G.d_h;
     A.h_h = (double*)G.h_h;
@@ -1933,6 +1949,7 @@ int bbhx_direct_like_fused(double* d_h, double* h_h, const double* data_freqs, c
     A.L = length;
     A.ntiles = ntiles;
     A.tile = tile;
+    A.block = (precision == 1) ? FD_TILE : tile;
     A.partials = part;
     A.segtab = segtab;
     A.d_h = d_h;
