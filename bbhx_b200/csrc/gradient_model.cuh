@@ -73,7 +73,7 @@ static __global__ void k_grad_setup(ModeCoeffsT<ad::Dual<N>>* coeffs, ResponseMo
     D fm, fs;
     final_mass_spin(m1, m2, chi1, chi2, &fm, &fs);
     // PhenomD 22 ringdown / damping from the tabulated spline (PhenomHMWaveform.cu:1930-1993)
-    const int ind = int((fs.v - (-1.0)) / dspin);
+    const int ind = qnm_row(fs.v, dspin, nq - 1);
     const D x = fs - (dspin * ind + (-1.0));
     const D x2 = x * x, x3 = x2 * x;
     const double* y_rd = qnm;

@@ -103,7 +103,7 @@ __global__ void k_count_point_ops(unsigned long long* out, const double* prm, co
   const double t_ref = prm[10];
   C fm, fs;
   final_mass_spin(m1, m2, chi1, chi2, &fm, &fs);
-  const int ind = int((fs.v + 1.0) / dspin);
+  const int ind = qnm_row(fs.v, dspin, nq - 1);
   const C x = fs - (dspin * ind - 1.0);
   const C x2 = x * x, x3 = x2 * x;
   const C rd22 = (qnm[ind] + qnm[nq + ind] * x + qnm[2 * nq + ind] * x2 + qnm[3 * nq + ind] * x3) / fm;

@@ -6,6 +6,7 @@
 // Layout of the waveform buffer (phenomhm.py:201-249): flat [nparams, B, M, L] with
 // slot 0 = amplitude, 1 = phase, 2 = t(f); freqs flat [B, M, L].
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "capi_internal.cuh"
@@ -32,13 +33,14 @@ __global__ void k_ringdown_d(double* fring, double* fdamp, const double* m1, con
                              const double* chi1, const double* chi2, int B, const double* y_rd,
                              const double* c1_rd, const double* c2_rd, const double* c3_rd,
                              const double* y_dm, const double* c1_dm, const double* c2_dm,
-                             const double* c3_dm, double dspin, int out_stride, int out_offset) {
+                             const double* c3_dm, double dspin, int last, int out_stride,
+                             int out_offset) {
   for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < B; b += gridDim.x * blockDim.x) {
     double fm, fs;
     final_mass_spin(m1[b], m2[b], chi1[b], chi2[b], &fm, &fs);
     double fr, fd;
-    phenomd_qnm_lookup(fs, fm, y_rd, c1_rd, c2_rd, c3_rd, y_dm, c1_dm, c2_dm, c3_dm, dspin, &fr,
-                       &fd);
+    phenomd_qnm_lookup(fs, fm, y_rd, c1_rd, c2_rd, c3_rd, y_dm, c1_dm, c2_dm, c3_dm, dspin, last,
+                       &fr, &fd);
     fring[(long long)b * out_stride + out_offset] = fr;
     fdamp[(long long)b * out_stride + out_offset] = fd;
   }
@@ -204,6 +206,8 @@ extern "C" {
 
 size_t bbhx_mode_coeffs_bytes(void) { return sizeof(ModeCoeffs); }
 
+int bbhx_selftest_qnm_row(double fs, double dspin, int last) { return qnm_row(fs, dspin, last); }
+
 // PhenomHMWaveform.hh:322-333
 int bbhx_get_phenomhm_ringdown_frequencies(double* fringdown, double* fdamp, const double* m1,
                                            const double* m2, const double* chi1z,
@@ -230,9 +234,11 @@ int bbhx_get_phenomd_ringdown_frequencies(double* fringdown, double* fdamp, cons
   BBHX_REQUIRE(num_bin_all >= 0, "num_bin_all < 0");
   BBHX_REQUIRE(dspin > 0.0, "dspin must be positive");
   if (num_bin_all == 0) return OK;
+  // the tables cover final spins -1 .. 1
+  const int last = (int)std::min(std::rint(2.0 / dspin), 2147483647.0);
   k_ringdown_d<<<grid_for(num_bin_all, kThreads), kThreads, 0, (cudaStream_t)stream>>>(
       fringdown, fdamp, m1, m2, chi1z, chi2z, num_bin_all, y_rd, c1_rd, c2_rd, c3_rd, y_dm, c1_dm,
-      c2_dm, c3_dm, dspin, 1, 0);
+      c2_dm, c3_dm, dspin, last, 1, 0);
   return launch_status("k_ringdown_d");
 }
 
@@ -261,7 +267,7 @@ int bbhx_ringdown_frequencies_all(double* fringdown, double* fdamp, const double
   k_ringdown_d<<<grid_for(num_bin_all, kThreads), kThreads, 0, s>>>(
       fringdown, fdamp, m1, m2, chi1z, chi2z, num_bin_all, T, T + table_len, T + 2 * table_len,
       T + 3 * table_len, T + 4 * table_len, T + 5 * table_len, T + 6 * table_len,
-      T + 7 * table_len, dspin, stride, off);
+      T + 7 * table_len, dspin, table_len - 1, stride, off);
   return launch_status("k_ringdown_d");
 }
 

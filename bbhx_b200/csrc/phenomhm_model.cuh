@@ -164,6 +164,14 @@ __device__ inline cplxT<T> qnm_cw(T jf, int ell, int mm) {
   return cmk(T(q.base + sum.re), sum.im);
 }
 
+// Row of the tabulated final-spin splines that holds fs, knots at -1 + k dspin, k = 0 .. last.  Held
+// to the table: the range check of the spins is read after the launches of a step, so this is also
+// evaluated for spins that the call then refuses (and for NaN, row 0).
+__host__ __device__ __forceinline__ int qnm_row(double fs, double dspin, int last) {
+  const double p = (fs - (-1.0)) / dspin;
+  return (p >= 1.0) ? ((p < (double)last) ? (int)p : last) : 0;
+}
+
 // Final spin (1508.07250 eq. 3.6) and radiated energy (eqs. 3.7-3.8); masses in any units
 // with m1 >= m2 enforced inside (PhenomHMWaveform.cu:1679-1814).
 template <typename T>

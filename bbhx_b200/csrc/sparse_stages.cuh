@@ -40,14 +40,15 @@ __device__ __forceinline__ void ringdown_hm(double m1, double m2, double chi1, d
 }
 
 // PhenomD 22 ringdown / damping frequency at final spin fs, final mass fm from the tabulated
-// final-spin splines (get_phenomd_ringdown_frequencies, PhenomHMWaveform.cu:1930-2062).
+// final-spin splines (get_phenomd_ringdown_frequencies, PhenomHMWaveform.cu:1930-2062); last = the
+// tables' last row.
 __device__ __forceinline__ void phenomd_qnm_lookup(double fs, double fm, const double* y_rd,
                                                    const double* c1_rd, const double* c2_rd,
                                                    const double* c3_rd, const double* y_dm,
                                                    const double* c1_dm, const double* c2_dm,
-                                                   const double* c3_dm, double dspin,
+                                                   const double* c3_dm, double dspin, int last,
                                                    double* fr, double* fd) {
-  int ind = int((fs - (-1.0)) / dspin);
+  const int ind = qnm_row(fs, dspin, last);
   double x = fs - (dspin * ind + (-1.0));
   double x2 = x * x, x3 = x2 * x;
   double r = y_rd[ind] + c1_rd[ind] * x + c2_rd[ind] * x2 + c3_rd[ind] * x3;
@@ -64,7 +65,7 @@ __device__ __forceinline__ void ringdown_d(double m1, double m2, double chi1, do
   double fm, fs;
   final_mass_spin(m1, m2, chi1, chi2, &fm, &fs);
   phenomd_qnm_lookup(fs, fm, T, T + nq, T + 2 * nq, T + 3 * nq, T + 4 * nq, T + 5 * nq,
-                     T + 6 * nq, T + 7 * nq, dspin, fr, fd);
+                     T + 6 * nq, T + 7 * nq, dspin, nq - 1, fr, fd);
 }
 
 // Point k of the default sparse grid (phenomhm.py:208-224): logspace(mf_min, mf_max, L) over

@@ -51,6 +51,9 @@ int bbhx_take_status(void *stream);
 int bbhx_pointer_is_device(const void *ptr);
 size_t bbhx_mode_coeffs_bytes(void);
 size_t bbhx_response_mode_bytes(void);
+/* self-test (no reference counterpart, host): the row 0 .. last of the ringdown tables that the
+ * kernels read for final spin fs (step dspin from -1) */
+int bbhx_selftest_qnm_row(double fs, double dspin, int last);
 /* self-test (no reference counterpart): out[4i..4i+3] = sin, cos of x[i] from the hot-loop
  * Cody-Waite + Taylor routine and from CUDA's sincos */
 int bbhx_selftest_sincos(const double *x, double *out, int n, void *stream);
