@@ -16,7 +16,7 @@ from . import _lib
 from .sensitivity import AET1SensitivityMatrix, SensitivityMatrix
 from .utils.arrays import device, to_dev, to_np, torch
 from .waveformbuild import PRECISIONS
-from .waveforms.phenomhm import raise_chi_flag
+from .waveforms.phenomhm import raise_chi_flag, raise_chi_range
 
 
 def pack_lnl(d_h, h_h, d_d, out=None):
@@ -339,15 +339,18 @@ class HeterodynedLikelihood:
         if self.precision is not None:
             kw = {k: v for k, v in waveform_kwargs.items()
                   if k in ("t_obs_start", "t_obs_end", "modes")}
-            self._last = (params, dict(waveform_kwargs))
-            self._h_sparse = None
-            # the spin check is read with the results: no synchronisation before the kernels
-            flags = t.empty(3, dtype=t.int32, device=device())
+            # spins out of range are refused before anything is launched or kept: parameters on the
+            # host are checked here, those on the device by step_front, which waits for its answer
+            flags = None
+            if not isinstance(params[0], t.Tensor):
+                raise_chi_range(params)
+                flags = t.empty(3, dtype=t.int32, device=device())
             self.hdyn_d_h, self.hdyn_h_h = self.template_gen.heterodyne_sums(
                 params, self.freqs, self._h0_flat, self.data_constants,
                 precision=self.precision, flags=flags, **kw)
+            self._last = (params, dict(waveform_kwargs))
+            self._h_sparse = None
         else:
-            flags = None
             self._h_sparse = self.template_gen(*params, **waveform_kwargs)
             r = self._h_sparse / self.h0_sparse
             B = r.shape[0]
@@ -358,14 +361,11 @@ class HeterodynedLikelihood:
                       _lib.dptr(residuals), _lib.dptr(self.data_constants), _lib.dptr(self.freqs),
                       B, len(self.freqs), 3, _lib.stream())
         B = self.hdyn_d_h.numel()
-        nf = 0 if flags is None else 3
-        packed_d = t.empty(3 * B + nf, dtype=t.float64, device=device())
+        packed_d = t.empty(3 * B, dtype=t.float64, device=device())
         _lib.call("bbhx_pack_lnl", _lib.dptr(packed_d), _lib.dptr(self.hdyn_d_h),
                   _lib.dptr(self.hdyn_h_h), float(self.reference_d_d), B,
-                  int(bool(phase_marginalize)), _lib.dptr(flags), nf, _lib.stream())
+                  int(bool(phase_marginalize)), _lib._VP(0), 0, _lib.stream())
         packed = packed_d.cpu().numpy()
-        if nf:
-            raise_chi_flag(int(packed[3 * B + 2]))
         out = packed[:B]
         if return_extracted_snr:
             return np.array([out, packed[B:2 * B] / np.sqrt(packed[2 * B:3 * B])]).T

@@ -51,6 +51,12 @@ def raise_chi_flag(code):
         raise ValueError(CHI2_MSG)
 
 
+def raise_chi_range(params):
+    """The same errors for parameter rows on the host (NaN passes, as in the kernel's check)."""
+    raise_chi_flag(sum(bit for row, bit in ((2, 1), (3, 2))
+                       if np.any(np.abs(params[row:row + 1]) > 1.0)))
+
+
 def step_front(m1, m2, chi1z, chi2z, lam=None, beta=None, num_modes=1, t_obs=(0.0, 0.0),
                flags=None):
     """Per-binary front end of a step in one kernel (bbhx_step_front): m1 >= m2 ordering with
