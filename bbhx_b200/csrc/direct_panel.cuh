@@ -447,7 +447,7 @@ __device__ __forceinline__ void panel_direct(const FusedArgs& A, cplx* gh, const
   __syncwarp();
 }
 
-// Bins [i0, i1) of binary b (inside its support) by one warp; kk = the segments of bins i0 and
+// Bins [i0, i1) of binary b (inside its support, i0 < i1) by one warp; kk = the segments of bins i0 and
 // i1 - 1 in lanes 0 .. M-1 (-1 before a mode's first knot, L-1 past its last).  Lane m walks mode
 // m.  When a mode enters segment k its freed ring slot is refilled with segment k + 3 by
 // asynchronous copies, three entries ahead of their use.  Per-lane partial sums into dr, di, hh;

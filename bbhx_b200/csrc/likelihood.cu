@@ -786,7 +786,8 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
     const int s0 = __ldg(A.sup_start + b);
     const int s1 = s0 + __ldg(A.sup_len + b);
     const int t0 = tile * A.tile;
-    if (t0 >= s1 || t0 + A.tile <= s0) {
+    const int i0 = max(t0, s0), i1 = min(t0 + A.tile, s1);  // the item's bins, none where i0 >= i1
+    if (i0 >= i1) {
       if (lane == 0) {
         double* P = A.partials + 3 * q;
         P[0] = 0.0; P[1] = 0.0; P[2] = 0.0;
@@ -797,8 +798,7 @@ __device__ __forceinline__ void fused_item(const FusedArgs& A, long long q, Warp
       if (uni) {
         const int2 kk = (lane < A.M) ? A.segtab[q * A.M + lane] : make_int2(0, 0);
         double dr = 0.0, di = 0.0, hh = 0.0;
-        panel_item<false>(A, *PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, gk0, gdf, dr, di,
-                          hh);
+        panel_item<false>(A, *PS, b, i0, i1, kk, lane, gk0, gdf, dr, di, hh);
         for (int o = 16; o > 0; o >>= 1) {
           dr += __shfl_xor_sync(0xffffffffu, dr, o);
           di += __shfl_xor_sync(0xffffffffu, di, o);
@@ -1186,10 +1186,11 @@ __global__ void __launch_bounds__(FD_WARPS * 32, 3) k_direct_panel(FusedArgs A) 
     const int b = (int)(q - (long long)tile * A.B);
     const int s0 = __ldg(A.sup_start + b), s1 = s0 + __ldg(A.sup_len + b);
     const int t0 = tile * A.tile;
+    const int i0 = max(t0, s0), i1 = min(t0 + A.tile, s1);
     double dr = 0.0, di = 0.0, hh = 0.0;
-    if (t0 < s1 && t0 + A.tile > s0) {
+    if (i0 < i1) {
       const int2 kk = (lane < A.M) ? A.segtab[q * A.M + lane] : make_int2(0, 0);
-      panel_item<GH>(A, PS, b, max(t0, s0), min(t0 + A.tile, s1), kk, lane, k0, df, dr, di, hh);
+      panel_item<GH>(A, PS, b, i0, i1, kk, lane, k0, df, dr, di, hh);
       for (int o = 16; o > 0; o >>= 1) {
         dr += __shfl_xor_sync(0xffffffffu, dr, o);
         di += __shfl_xor_sync(0xffffffffu, di, o);
