@@ -114,13 +114,14 @@ class DirectGroup:
         tab = ap.qnm_table
         self._keep = (x, y, c1, c2, c3, ts, te, ells, mms, tab)
         p = lambda a: _lib.dptr(a).value if a is not None else None  # noqa: E731
+        tmin, tmax = rg.t_span
         return DirectSourceC(
             orbits=rg.orbit_handle.ptr.value, params=p(self.params), ells=p(ells), mms=p(mms),
             qnm_table=p(tab), qnm_n=int(tab.shape[1]), dspin=float(dspin),
             mf_min=float(ap.mf_min), mf_max=float(ap.mf_max), t_init=float(ap.initial_t_val),
             t_obs_start_L=float(self.t_obs_start * YRSID_SI),
             t_obs_end_L=float(self.t_obs_end * YRSID_SI),
-            orbit_tmin=float(rg.orbits.t_base.min()), orbit_tmax=float(rg.orbits.t_base.max()),
+            orbit_tmin=tmin, orbit_tmax=tmax,
             TDItag=rg.TDItag_int, rescaled=int(rg.rescaled), tdi2=int(rg.tdi2),
             run_phenomd=int(ap.run_phenomd), num_modes=M, length=L, num_bin_all=B, x=p(x),
             y=p(y), c1=p(c1), c2=p(c2), c3=p(c3), t_start=p(ts), t_end=p(te),
