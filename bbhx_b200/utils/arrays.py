@@ -43,6 +43,8 @@ def param_rows(params):
     call); anything else is converted one by one.  f_ref (6) does not enter the model and is passed
     through."""
     t = torch()
+    if len(params) != 12:
+        raise ValueError("12 source parameters are needed, got %d" % len(params))
     if not any(isinstance(v, t.Tensor) for v in params):
         rows = [np.atleast_1d(np.asarray(v)) for k, v in enumerate(params) if k != 6]
         if all(r.ndim == 1 and r.shape == rows[0].shape and r.dtype.kind in "fiub" for r in rows):
