@@ -292,7 +292,7 @@ __global__ void k_spline_adj(double* ybar, double* xbar, const double* ybd, cons
       }
     }
     __syncthreads();
-    cr_solve(a, bb, c, w, d, 9, L);  // lambda = K^{-T} s_bar (r_bar)
+    cr_solve<false>(a, bb, c, w, d, 9, L);  // lambda = K^{-T} s_bar (r_bar)
     // y_bar from m_bar
     for (int i = threadIdx.x; i < L; i += blockDim.x) {
       for (int p = 0; p < 9; ++p) {

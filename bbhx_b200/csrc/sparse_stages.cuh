@@ -287,7 +287,7 @@ __device__ inline void spline_system_t(const double* xg, const double* y, long l
   // keep the last row's matrix entries for the c1/c2/c3[L-1] convention
   const double last_a = a[cr_slot(L - 1)], last_b = b[cr_slot(L - 1)];
   __syncthreads();
-  cr_solve(a, b, c, w, d, P, L);
+  cr_solve<PT == 0>(a, b, c, w, d, P, L);  // nine quantities: no block has 18 warps
   for (int i = threadIdx.x; i < L; i += blockDim.x) {
     const bool seg = i < L - 1;
     const double ih = seg ? 1.0 / (xg[i + 1] - xg[i]) : 1.0;

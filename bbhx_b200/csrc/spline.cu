@@ -45,6 +45,19 @@ using namespace bbhx;
 
 namespace {
 constexpr size_t kMaxSplineSmem = 204 * 1024;
+
+// Threads of a block (126 registers each: 512 to an SM).  A block with an SM of its own, because the
+// systems are few or long, is bound by the latency of its levels and takes twelve warps (1024 knots
+// x 9 quantities, six systems: 40 us, 48 with eight warps; 2000 x 9, 600 systems: 277 and 346).
+// Many systems are bound by throughput: short ones take few warps, since a level of 32 rows or fewer
+// occupies one, and more blocks share the SM.  With eight warps, with the length's:
+//   64 x 1, 100,000 systems 2674, 493 us       128 x 9, 24,000 systems 1198, 739 us
+//   300 x 4, 20,000 systems 1089, 650 us       512 x 9, 5,400 systems 542, 468 us
+//   1024 x 9, 6144 systems 1035 us (four warps 1383, nine, one block per SM, 1345)
+int spline_threads(int length, long long systems, size_t smem, bool use_smem) {
+  if (systems <= sm_count() || !use_smem || smem > 110 * 1024) return 384;
+  return length <= 64 ? 32 : length <= 320 ? 64 : length <= 700 ? 128 : 256;
+}
 }
 
 extern "C" {
@@ -61,7 +74,7 @@ int bbhx_interpolate(const double* freqs, const double* y, double* B_, double* u
   cudaStream_t s = (cudaStream_t)stream;
   size_t smem = sizeof(double) * spline_work(length, num_interp_params);
   bool use_smem = smem <= kMaxSplineSmem;
-  int threads = 288;  // nine warps: one right-hand side each of the sparse buffer's nine
+  const int threads = spline_threads(length, S, smem, use_smem);
   const long long nsm = sm_count();
   unsigned int grid = (unsigned int)(S < nsm * 16 ? S : nsm * 16);
   double* scratch = nullptr;
