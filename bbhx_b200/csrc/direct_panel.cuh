@@ -565,6 +565,8 @@ __device__ __forceinline__ void panel_item(const FusedArgs& A, PanelStage& PS, i
         ++k;
         enter();
       }
+      // the segment just entered has been read before the next round's copies may take its slot
+      __syncwarp();
       move = __ballot_sync(0xffffffffu, go && k < L - 1 && next <= i);
     }
     __syncwarp();
