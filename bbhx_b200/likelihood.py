@@ -334,16 +334,20 @@ class HeterodynedLikelihood:
             if params.ndim == 1:
                 params = params.reshape(-1, 1)
             params = tuple(params[k].contiguous() for k in range(params.shape[0]))
+            spins = None
         else:
-            params = tuple(np.atleast_2d(np.asarray(params, dtype=np.float64)))
+            params = np.atleast_2d(np.asarray(params, dtype=np.float64))
+            spins = params[2:4]
+            params = tuple(params)
         if self.precision is not None:
             kw = {k: v for k, v in waveform_kwargs.items()
                   if k in ("t_obs_start", "t_obs_end", "modes")}
-            # spins out of range are refused before anything is launched or kept: parameters on the
-            # host are checked here, those on the device by step_front, which waits for its answer
+            # spins out of range are refused before anything is launched or kept: on the host where
+            # the parameters are there and few (8 us up to some thousand walkers, 20 at 16384, 63 at
+            # 65536), else by step_front, which waits for the device's answer (15-20 us)
             flags = None
-            if not isinstance(params[0], t.Tensor):
-                raise_chi_range(params)
+            if spins is not None and spins.size <= 2 * 16384:
+                raise_chi_range(spins)
                 flags = t.empty(3, dtype=t.int32, device=device())
             self.hdyn_d_h, self.hdyn_h_h = self.template_gen.heterodyne_sums(
                 params, self.freqs, self._h0_flat, self.data_constants,

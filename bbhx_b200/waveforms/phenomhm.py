@@ -51,10 +51,11 @@ def raise_chi_flag(code):
         raise ValueError(CHI2_MSG)
 
 
-def raise_chi_range(params):
-    """The same errors for parameter rows on the host (NaN passes, as in the kernel's check)."""
-    raise_chi_flag(sum(bit for row, bit in ((2, 1), (3, 2))
-                       if np.any(np.abs(params[row:row + 1]) > 1.0)))
+def raise_chi_range(spins):
+    """The same errors for the rows chi1z, chi2z of an array on the host (NaN passes, as in the
+    kernel's check)."""
+    if spins.size and not (spins.max() <= 1.0 and spins.min() >= -1.0):
+        raise_chi_flag(sum(bit for bit, row in zip((1, 2), spins) if np.any(np.abs(row) > 1.0)))
 
 
 def step_front(m1, m2, chi1z, chi2z, lam=None, beta=None, num_modes=1, t_obs=(0.0, 0.0),

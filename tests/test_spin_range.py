@@ -56,10 +56,22 @@ def test_heterodyned_refuses_spins_before_any_launch(row, value, message):
     assert (het.hdyn_d_h, het.hdyn_h_h, het._last, het._h_sparse) == ("d_h", "h_h", "last", "sparse")
 
 
+def test_nan_spins_pass_and_hide_nothing():
+    from bbhx_b200.waveforms.phenomhm import raise_chi_range
+
+    spins = np.array([[0.1, np.nan, -1.0], [1.0, np.nan, 0.3]])
+    raise_chi_range(spins)
+    raise_chi_range(spins[:, :0])
+    spins[1, 2] = -1.5
+    with pytest.raises(ValueError, match="chi2z"):
+        raise_chi_range(spins)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
-@pytest.mark.parametrize("on_device", [False, True])
-def test_heterodyned_is_as_before_after_a_refused_call(golden, golden_data, precision, on_device):
+@pytest.mark.parametrize("on_device,copies", [(False, 1), (True, 1), (False, 2100)])
+def test_heterodyned_is_as_before_after_a_refused_call(golden, golden_data, precision, on_device,
+                                                       copies):
     import torch
 
     from bbhx_b200 import AET1SensitivityMatrix, BBHWaveformFD, EqualArmlengthOrbits
@@ -71,7 +83,7 @@ def test_heterodyned_is_as_before_after_a_refused_call(golden, golden_data, prec
                                 template_gen_kwargs=dict(kw), reference_gen_kwargs=dict(kw, length=1024),
                                 sens_mat=AET1SensitivityMatrix(golden_data["f"], tdi2=True),
                                 precision=precision)
-    P = golden["het_walkers"]
+    P = np.tile(golden["het_walkers"], (1, copies))  # 8 walkers; 16800 are checked on the device
     as_given = (lambda a: torch.as_tensor(a, device="cuda")) if on_device else (lambda a: a)
     ref = het.get_ll(as_given(P), **kw).copy()
     d_h, last = het.hdyn_d_h.clone(), het._last
