@@ -231,7 +231,7 @@ template <typename R>
 constexpr int fd_nseg() { return sizeof(R) == 8 ? 4 : 8; }
 constexpr int FD_MAXM = 6;    // modes per binary
 constexpr int FD_NC = 36;     // 9 quantities x (y, c1, c2, c3) per segment
-constexpr int FD_MAXCHUNK = 32;  // 128-bin chunks per tile item (tiles of up to 4096 bins)
+constexpr int FD_MAXCHUNK = 32;  // 128-bin chunks of an FD_TILE (FP64 single-problem items: twice)
 
 struct FusedArgs {
   const double* data_freqs;
@@ -504,7 +504,7 @@ struct alignas(16) WarpStage {
 // frequency k df (error-free product) with a compensated final sum, so it carries < 1e-13 rad
 // instead of the ~ulp(phi) ~ 1e-10 - 1e-9 rad of a plain FP64 evaluation, and the products add
 // ~2e-11 rad over 128 steps.  No likelihood kernel runs it (the panels of direct_panel.cuh took
-// its place, with the same anchor arithmetic at their nodes); bbhx_selftest_recurrence does.
+// its place); bbhx_selftest_recurrence does.
 struct Rot {
   double er, ei, rr, ri, qr, qi, pr, pi;
 };
@@ -1426,7 +1426,10 @@ unsigned resident_grid(K kernel, size_t smem, long long nitems) {
 // Data bins per work item of a single-problem launch: the largest tile up to `tile` that still
 // gives every resident warp several items, since an item of a low-frequency tile takes many times
 // the average and the call ends when its slowest item does (call with B = 1, 1 yr: 1.81 ms at 4096
-// bins, 0.86 ms at 512; B = 1024: 1.1 ms less at 8192 bins than at 4096).
+// bins, 0.86 ms at 512; B = 1024: 1.1 ms less at 8192 bins than at 4096).  The mixed form, four CTAs
+// per SM, up to 4096 bins: B = 1, 1 yr 1.48 ms at 4096 bins, 0.55 ms with its own size; B = 69 at
+// 0.15 yr 1.19 and 0.85 ms.  Non-uniform grids in FP64: B = 1, 1 yr 1.70 and 0.60 ms, B = 400 (8192
+// bins) 55.2 and 52.2 ms.
 inline int fused_tile(int N, int B, int tile) {
   const long long warps = (long long)sm_count() * 3 * FD_WARPS;
   while (tile > 256 && ((long long)N + tile - 1) / tile * B < 8 * warps) tile >>= 1;
