@@ -13,8 +13,9 @@ and sums; FP32 amplitude and transfer) is timed beside it with its |dlnL| agains
   value  : FP64 lnL evaluations / s with parameters already resident on the GPU
   e2e    : the same through the public API (Likelihood.get_ll) from pinned host params,
            including the H2D copy of the 12 x B parameters and the D2H copy of the B lnL
-  roofline: the fused FP64 interpolate + reduce kernel against measured HBM bandwidth, with
-           72 B of algorithmic traffic per (binary, data bin) (the FP64 data and weights)
+  roofline: the fused FP64 interpolate + reduce kernel against the FP64 pipe, with the 70
+           instructions per (binary, data bin) it cannot do without; its 72 B of data and weights
+           per pair against measured HBM bandwidth (`hbm`) are no bound: they are L2-resident
   cpu_baseline: the reference's own C++ CPU path (oracle/_ref) on a bounded sample
 
 Usage: python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
@@ -42,9 +43,9 @@ SEED_NOISE = 99
 HBM_BYTES_PER_PAIR = 72.0  # 3 x complex128 weighted data + 3 x float64 noise weights
 MIXED_BYTES_PER_PAIR = 36.0  # 3 x complex64 + 3 x float32: the FP32 copies the mixed form reads
 # FP64 instructions per (binary, bin) pair the panel form cannot do without, whatever the number of
-# modes: per channel a complex polynomial of degree 7 (14), the carrier product (4), and the products
-# with weight and data (8)
-FP64_INSTR_PER_PAIR = 3 * (14 + 4 + 8)
+# modes: per channel a complex polynomial of degree 7 (14) and the products with weight and data
+# (8), and one carrier product for the three (4)
+FP64_INSTR_PER_PAIR = 3 * (14 + 8) + 4
 # the library's kernels in one direct step (ncu launch list): k_clear_flags, k_step_front,
 # k_ringdown_hm, k_ringdown_d, k_phm_setup, k_default_freqs, k_phm_tf, k_tf_window,
 # k_response_setup, k_phm_response, k_tf_range, k_spline, k_support, k_grid_detect,
@@ -416,14 +417,15 @@ def gpu_arm(args):
                 "h2d_bytes_per_step": 12 * B * 8, "d2h_bytes_per_step": 3 * B * 8 + 3 * 8,
                 "path": "Likelihood.get_ll (precision='fp64') from pinned host parameters",
                 "max_abs_dlnl_vs_device_path": dl},
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak,
-                     "algorithmic_bytes_per_pair": HBM_BYTES_PER_PAIR,
-                     "traffic": (tpp * pairs if tpp is not None else None),
+        "roofline": {**fp64_roofline(pairs, fused_avg_s),
                      "kernel": "k_direct_panel (bbhx_direct_like_fused, precision 0)",
                      "kernel_ms": statistics.mean(fused_ms),
-                     "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if peaks else "fallback",
-                     "fp64_floor": fp64_floor(pairs, fused_avg_s, peak)},
+                     "traffic": (tpp * pairs if tpp is not None else None),
+                     "hbm": {"achieved": achieved, "peak": peak, "unit": "GB/s",
+                             "frac": achieved / peak,
+                             "algorithmic_bytes_per_pair": HBM_BYTES_PER_PAIR,
+                             "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)"
+                                            if peaks else "fallback"}},
         "gpu_launches": LAUNCHES_PER_STEP * args.steps,
         "clocks": clocks,
     }
@@ -570,16 +572,15 @@ OPC_NAMES = ("add_sub", "mul", "div", "compare", "sqrt", "cbrt", "log", "exp", "
              "sin_cos", "other")
 
 
-def fp64_floor(pairs, kernel_s, hbm_peak_gbs):
+def fp64_roofline(pairs, kernel_s):
     """The FP64 pipe's bound on the direct kernel: FP64_INSTR_PER_PAIR instructions for every pair
     (the panels' nodes and the bins evaluated one by one come on top) at the nominal FP64 lane rate
-    give the shortest possible kernel time, and the HBM-roofline fraction the kernel would reach
-    there."""
-    floor_s = FP64_INSTR_PER_PAIR * pairs / fp64_lane_rate()
-    return {"fp64_instr_per_pair": FP64_INSTR_PER_PAIR, "floor_ms": floor_s * 1e3,
-            "kernel_over_floor": kernel_s / floor_s,
-            "hbm_frac_at_floor": HBM_BYTES_PER_PAIR * pairs / floor_s / 1e9 / hbm_peak_gbs,
-            "lane_rate": "the device's SMs x 64 FP64 lanes x 1965 MHz (nominal clock)"}
+    give the shortest possible kernel time."""
+    work, peak = FP64_INSTR_PER_PAIR * pairs, fp64_lane_rate()
+    return {"bound": "fp64", "achieved": work / kernel_s / 1e12, "peak": peak / 1e12,
+            "unit": "T FP64 instructions/s", "frac": work / kernel_s / peak,
+            "fp64_instr_per_pair": FP64_INSTR_PER_PAIR, "floor_ms": work / peak * 1e3,
+            "peak_source": "the device's SMs x 64 FP64 lanes x 1965 MHz (nominal clock)"}
 
 
 def het_roofline(het, wave, center, evals_per_s):
