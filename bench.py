@@ -824,7 +824,11 @@ def reference_arm(args):
         return None
     from bbhx_b200.synthetic import data_grid
     from bbhx_b200.synthetic import draw_params
+    from oracle.build_ref import OUT
 
+    if not os.path.exists(OUT):
+        return {"impl": "reference",
+                "unavailable": "the reference's CPU library is not built (oracle/build_ref.py)"}
     params = draw_params(args.batch, TOBS, SEED_PARAMS)
     workers = cpu_workers()
     val, times = cpu_reference(params, workers, steps=args.steps, warmup=args.warmup)
